@@ -175,11 +175,14 @@ void free_table(s615_ctx* ctx, DevTable& t) {
   dev_free(ctx, t.d_cells, t.bytes);
   t.d_cells = nullptr;
   t.bytes = 0;
+  dev_free(ctx, t.d_plane, t.plane_bytes);
+  t.d_plane = nullptr;
+  t.plane_bytes = 0;
 }
 
 // Device bytes of a table or of every shard of a set.
 size_t table_bytes(const DevTable& t) {
-  size_t b = t.bytes;
+  size_t b = t.bytes + t.plane_bytes;
   for (const DevTable& p : t.parts) b += p.bytes;
   return b;
 }
@@ -559,6 +562,7 @@ int s615_load_table(s615_ctx* ctx, const char* path, int expected_N, int layout,
   int s = load_part(ctx, path, expected_N, layout, &t);
   if (s) return s;
   if (t.hdr.shard_count != 1) { free_table(ctx, t); return S615_E_FORMAT; }   // one shard of a set
+  if ((s = build_plane(ctx, t, ctx->stream))) { free_table(ctx, t); return s; }
   int id = 0;
   add_table(ctx, t, &id);
   if ((s = smoke_table(ctx, id))) { s615_free_table(ctx, id); return s; }
@@ -708,6 +712,7 @@ int s615_build_table(s615_ctx* ctx, int N, int r, int layout, int* table_id) {
                        layout == S615_LAYOUT_AUTO ? S615_LAYOUT_WIDE : layout, &t);
   dev_free(ctx, dv, vals.size() * 8);
   if (s) return s;
+  if ((s = build_plane(ctx, t, ctx->stream))) { free_table(ctx, t); return s; }
   int id = 0;
   add_table(ctx, t, &id);
   if ((s = smoke_table(ctx, id))) { s615_free_table(ctx, id); return s; }
@@ -774,6 +779,7 @@ int s615_build_table_keys(s615_ctx* ctx, const uint64_t* keys, size_t n, int r, 
                        layout == S615_LAYOUT_AUTO ? S615_LAYOUT_WIDE : layout, &t);
   dev_free(ctx, dk, std::max<size_t>(n, 1) * 8);
   if (s) return s;
+  if ((s = build_plane(ctx, t, ctx->stream))) { free_table(ctx, t); return s; }
   return add_table(ctx, t, table_id);
 }
 

@@ -97,6 +97,11 @@ struct DevTable {
   u32 shard_lo = 0;              // parts[i] is shard shard_lo + i of hdr.shard_count
   void* d_views = nullptr;       // one TableView per shard of the set in HBM (owned ones set)
   u32 groups = 0;                // probe passes over a set (0: from its size)
+  // The plane: the low 2^plane_lb bits of every cell, packed into 32-bit words
+  // (a single table whose plane fits L2 far better than its cells; table.cu).
+  void* d_plane = nullptr;
+  size_t plane_bytes = 0;
+  u32 plane_lb = 0;
 };
 
 // Random reads keep their rate over footprints up to 64 GiB and lose ~3x at
@@ -118,6 +123,9 @@ struct TableView {
   u32 grp_lo, grp_hi;   // this pass probes keys of shards [grp_lo, grp_hi)
   u32 groups, pad;      // passes over the set
   u64 bytes;            // bytes of cells (a single table; 0 for a set)
+  const u32* plane;     // low 2^plane_lb bits of each cell (null: none)
+  u64 plane_bytes;
+  u32 plane_lb, plane_mask;   // plane_mask = 2^(2^plane_lb) - 1
 };
 
 struct Cls5Counters {  // device accumulators (u64 atomics)
@@ -299,6 +307,9 @@ int launch_peel(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flag
                 cudaStream_t st, int grid_blocks);
 int launch_peel617(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                    cudaStream_t st, int grid_blocks);
+// Builds t's plane when it would make the probe cheaper (and the HBM budget
+// has room for it); a table without one is probed through its cells alone.
+int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st);
 int launch_xor_query(s615_ctx* ctx, const TableView& tv, const u64* d_keys, size_t n,
                      u8* d_out, cudaStream_t st);
 int launch_unpack(s615_ctx* ctx, const u8* d_packed, u64 m, u32 r, void* d_wide, int cell_bytes,

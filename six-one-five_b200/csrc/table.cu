@@ -61,6 +61,35 @@ __global__ void k_pack(const Cell* __restrict__ wide, u64 m, u32 r,
   }
 }
 
+// One thread per 32-bit plane word: the low 2^lb bits of its 32 >> lb cells.
+__global__ void k_plane(const void* __restrict__ cells, u32 layout, u32 cell_bytes, u32 r, u64 m,
+                        u32 lb, u32* __restrict__ plane, u64 n_words) {
+  const u32 per = 32u >> lb, bits = 1u << lb;
+  const u32 mask = (u32)((1ull << bits) - 1);
+  for (u64 w = blockIdx.x * (u64)blockDim.x + threadIdx.x; w < n_words;
+       w += (u64)gridDim.x * blockDim.x) {
+    const u64 c0 = w * per;
+    u32 word = 0;
+    for (u32 k = 0; k < per && c0 + k < m; ++k)
+      word |= ((u32)load_cell_at(cells, layout, cell_bytes, r, fp_mask(r), c0 + k) & mask) << (k * bits);
+    plane[w] = word;
+  }
+}
+
+// Picoseconds per scattered read over a footprint, the whole GPU reading
+// (measured on a B200: 2.85e11 reads/s up to 64 MB, 4.71e10 /s at 28 GB).
+double read_ps(double mb) {
+  static const double at[][2] = {{64, 3.5},   {80, 4.25},  {96, 6.2},    {112, 8.1},   {128, 9.6},
+                                 {160, 11.7}, {192, 13.0}, {256, 14.7},  {384, 16.3},  {512, 17.1},
+                                 {1024, 18.5}, {2048, 19.7}, {4096, 20.4}, {8192, 21.1}};
+  constexpr int n = sizeof at / sizeof at[0];
+  if (mb <= at[0][0]) return at[0][1];
+  for (int i = 1; i < n; ++i)
+    if (mb <= at[i][0])
+      return at[i - 1][1] + (at[i][1] - at[i - 1][1]) * (mb - at[i - 1][0]) / (at[i][0] - at[i - 1][0]);
+  return at[n - 1][1];
+}
+
 int grid_for(s615_ctx* ctx, u64 n, int threads) {
   const u64 want = (n + threads - 1) / threads;
   const u64 cap = (u64)ctx->num_sms * 16;
@@ -97,8 +126,56 @@ TableView view_of(const DevTable& t) {
   v.r = t.hdr.r;
   v.layout = (u32)t.layout;
   v.cell_bytes = (u32)t.cell_bytes;
+  v.plane = static_cast<const u32*>(t.d_plane);
+  v.plane_bytes = t.plane_bytes;
+  v.plane_lb = t.plane_lb;
+  v.plane_mask = (u32)((1ull << (1u << t.plane_lb)) - 1);
   if (t.hdr.n_keys == 0 || t.hdr.m_cells < 3) v.block = 0;
   return v;
+}
+
+// A probe costs three scattered reads of cells, or with a plane of b bits
+// three reads of the plane and, for 2^-b of the probes, three of cells.  The
+// widths tried are 1, 2, 4 and 8 bits, up to 112 MB; the cheapest by read_ps
+// is taken when it saves a tenth.  Past 112 MB (N above about 39,000 at one
+// bit) the plane is mostly read from DRAM itself: a 4-bit plane of 468 MB gave
+// a class-5 pass 7% and took 14% from a mixed one.  Measured, ps per probe
+// through the cells alone / with the plane: class 5, N = 12,000 (4 bits) 65.5
+// / 43.6, 20,000 (2 bits) 63.2 / 34.4, 24,000 (2 bits) 63.2 / 38.1, 31,000 (1
+// bit) 63.1 / 46.5, 37,000 (1 bit) 63.2 / 54.4; (6,1,7), N = 10,476 (8 bits) 54.7 /
+// 14.6.  Three reads of a 64 MB plane are 10.5 ps.
+constexpr double kPlaneMaxMB = 112;
+int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
+  const u64 m = t.hdr.m_cells;
+  if (!t.d_cells || t.hdr.n_keys == 0 || m < 3) return S615_OK;
+  const double cell_ps = 3 * read_ps((double)t.bytes / 1048576.0);
+  double best = 0.9 * cell_ps;
+  int lb = -1;
+  for (int k = 0; k < 4; ++k) {
+    const u32 bits = 1u << k;
+    if (bits > t.hdr.r) break;
+    const double mb = (double)m * bits / 8 / 1048576.0;
+    const double ps = 3 * read_ps(mb) + cell_ps / (double)(1u << bits);
+    if (mb <= kPlaneMaxMB && ps < best) { best = ps; lb = k; }
+  }
+  if (lb < 0) return S615_OK;
+  const u32 per = 32u >> lb;
+  const u64 words = (m + per - 1) / per;
+  void* p = nullptr;
+  if (dev_alloc(ctx, &p, words * sizeof(u32))) return S615_OK;   // no room: the cells alone
+  k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
+                                                     t.hdr.r, m, (u32)lb, static_cast<u32*>(p), words);
+  ctx->launches++;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    dev_free(ctx, p, words * sizeof(u32));
+    return cuda_status(e);
+  }
+  t.d_plane = p;
+  t.plane_bytes = words * sizeof(u32);
+  t.plane_lb = (u32)lb;
+  return S615_OK;
 }
 
 int launch_xor_query(s615_ctx* ctx, const TableView& tv, const u64* d_keys, size_t n,
