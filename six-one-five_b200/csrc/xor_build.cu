@@ -7,8 +7,9 @@
 //  1. Key set.  Pair mode enumerates unordered pairs of the DISTINCT values
 //     of i^6 mod 2^64 (1<=i<=N); many i share a value (every multiple of 2048
 //     has i^6 = 0 mod 2^64), so this already removes most duplicate keys.
-//     Remaining duplicates are removed by an open-addressing hash set in HBM
-//     (the reference sorts + uniques).  The survivors are the unique keys.
+//     The keys are partitioned by mix64(key) into slices whose hash set stays
+//     in L2, and each slice's duplicates are removed there (the reference
+//     sorts + uniques).  The survivors are the unique keys.
 //  2. Incidence: every cell is one 64-bit word, count << 42 | sum of the
 //     indices of its keys, and each key adds (1 << 42) + index to its three
 //     cells (binned by L2-sized cell slice when HBM allows).
@@ -57,85 +58,317 @@ int grid_for(s615_ctx* ctx, u64 n, int threads) {
   return (int)(want < cap ? (want ? want : 1) : cap);
 }
 
-__device__ __forceinline__ void hset_insert(unsigned long long* table, u64 tmask, u64 key,
-                                            u32* has_empty_key) {
-  if (key == kEmpty) { *has_empty_key = 1; return; }
-  u64 pos = mix64(key ^ 0x5bd1e9955bd1e995ULL) & tmask;
-  for (u64 probe = 0; probe <= tmask; ++probe) {
-    const unsigned long long old = atomicCAS(table + pos, (unsigned long long)kEmpty,
-                                             (unsigned long long)key);
-    if (old == kEmpty || old == key) return;
-    pos = (pos + 1) & tmask;
-  }
+// Blocks for n items at `per` items a block.  The kernels that read or update
+// random cells take one small tile per block: the block scheduler then hands
+// tiles out as SMs become free.  Scattered accesses are served per group of 2
+// to 8 SMs at an equal rate per group, so a static split waits for the largest
+// groups (random reads over 28 GB: 3.65e10/s split evenly, 4.71e10/s dealt out).
+u32 blocks_for(u64 n, u64 per) {
+  const u64 b = (n + per - 1) / per;
+  return (u32)std::min<u64>(std::max<u64>(b, 1), 0x7FFFFFFFull);
 }
 
-// Which keys this build takes: the memory partition (top bits of mix64(key))
-// and, for one shard of a set, mix64(key + kShardSeed) % shards == shard.
-struct KeyFilter {
-  u32 part_bits, part, shards, shard;
-  u64 srecip;
-  __device__ __forceinline__ bool take(u64 key) const {
-    if (part_bits && (mix64(key) >> (64 - part_bits)) != part) return false;
-    return shards <= 1 || fast_mod(mix64(key + kShardSeed), shards, srecip) == shard;
-  }
-};
-
-// Pair keys u[a] + u[b], a <= b, one block-stride row per a.
-__global__ void k_insert_pairs(const u64* __restrict__ vals, u64 nv, unsigned long long* table,
-                               u64 tmask, KeyFilter kf, u32* has_empty_key) {
-  for (u64 a = blockIdx.x; a < nv; a += gridDim.x) {
-    const u64 va = vals[a];
-    for (u64 b = a + threadIdx.x; b < nv; b += blockDim.x) {
-      const u64 key = va + vals[b];
-      if (kf.take(key)) hset_insert(table, tmask, key, has_empty_key);
-    }
-  }
-}
-
-__global__ void k_insert_keys(const u64* __restrict__ keys, u64 n, unsigned long long* table,
-                              u64 tmask, KeyFilter kf, u32* has_empty_key) {
-  for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < n;
-       i += (u64)gridDim.x * blockDim.x) {
-    const u64 key = keys[i];
-    if (kf.take(key)) hset_insert(table, tmask, key, has_empty_key);
-  }
-}
-
-// Append occupied slots to out (order irrelevant); slots past cap are
-// counted, not written.
-// The flagged threads' positions in a list whose length is *count, with ONE
-// global atomic per block (a shared-memory scan of the warps' counts): the
-// lists' counters are single addresses, and per-warp atomics on them
-// serialise in their L2 slice.  Every thread of the block calls this (it
-// synchronises the block); ~0 for a thread that takes nothing.
-__device__ __forceinline__ u64 block_reserve(bool take, unsigned long long* count) {
+// Positions of the flagged items in a list whose length is *count, K per
+// thread, with ONE global atomic per block (a shared-memory scan of the warps'
+// counts): the lists' counters are single addresses, and per-warp atomics on
+// them serialise in their L2 slice (~1.7e8/s; the peel of N = 76,667 took 1,554
+// ms with them, 711 ms per block).  Every thread of the block calls this (it
+// synchronises the block); pos[k] is set where take[k] is.
+template <int K>
+__device__ __forceinline__ void block_positions(const bool (&take)[K], unsigned long long* count,
+                                                u64 (&pos)[K]) {
   __shared__ u32 s_cnt[32];
   __shared__ unsigned long long s_base;
   const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  const u32 b = __ballot_sync(0xFFFFFFFFu, take);
+  u32 b[K];
+  u32 wtot = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    b[k] = __ballot_sync(0xFFFFFFFFu, take[k]);
+    wtot += __popc(b[k]);
+  }
   __syncthreads();   // the previous call's offsets have been read
-  if (lane == 0) s_cnt[wid] = __popc(b);
+  if (lane == 0) s_cnt[wid] = wtot;
   __syncthreads();
   if (threadIdx.x == 0) {
     u32 tot = 0;
     for (u32 w = 0; w < nw; ++w) {
-      const u32 k = s_cnt[w];
+      const u32 n = s_cnt[w];
       s_cnt[w] = tot;
-      tot += k;
+      tot += n;
     }
     s_base = tot ? atomicAdd(count, (unsigned long long)tot) : 0ull;
   }
   __syncthreads();
-  return take ? s_base + s_cnt[wid] + __popc(b & ((1u << lane) - 1u)) : ~0ull;
+  u64 at = s_base + s_cnt[wid];
+  const u32 below = (1u << lane) - 1u;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    pos[k] = at + __popc(b[k] & below);
+    at += __popc(b[k]);
+  }
 }
 
-__global__ void k_compact(const unsigned long long* __restrict__ table, u64 tsize,
-                          u64* __restrict__ out, u64 cap, unsigned long long* n_out) {
-  for (u64 i0 = blockIdx.x * (u64)blockDim.x; i0 < tsize; i0 += (u64)gridDim.x * blockDim.x) {
-    const u64 i = i0 + threadIdx.x;
-    const bool occ = i < tsize && table[i] != kEmpty;
-    const u64 k = block_reserve(occ, n_out);   // every thread of the block, every pass
-    if (occ && k < cap) out[k] = table[i];
+// ---- partition through shared memory ----------------------------------------
+// Items (8 B each) are sorted by slice in two passes over the same source.
+// k_part_count counts each block's items per slice in shared memory; a scan
+// over (slice, block) gives every block its own output range per slice;
+// k_part_scatter then takes tiles of kTile items, orders a tile by slice in
+// shared memory and writes each slice's run with consecutive threads.  Writing
+// items one by one was bound by the rate of scattered stores (2e10/s: 150 of
+// the 219 ms of the N = 48,000 incidence); runs of 5 to 12 items divide the
+// store requests accordingly.
+constexpr u32 kMaxSlices = 4608;
+constexpr int kPartThreads = 512;
+constexpr int kPartPer = 16;
+constexpr u32 kTile = kPartThreads * kPartPer;   // items per tile: 64 KB staged
+
+// Source of the key partition: the t-th raw key, t < n.  Pairs are numbered
+// along rows a and nv - 1 - a laid end to end (nv + 1 pairs together), so a
+// flat range of t has no short rows.
+struct KeySource {
+  const u64* vals;   // pair mode: distinct values; null: keys
+  const u64* keys;
+  u64 nv, n, row_recip;
+  u32 shards, shard;
+  u64 srecip;
+  u32 S, s_lo, s_hi;   // slices in all, and those this pass takes
+  __device__ __forceinline__ u64 key(u64 t) const {
+    if (!vals) return keys[t];
+    const u64 len = nv + 1;
+    u64 p = mulhi64(t, row_recip), q = t - p * len;   // p is at most 2 short
+    if (q >= len) { q -= len; ++p; }
+    if (q >= len) { q -= len; ++p; }
+    const u64 first = nv - p;
+    const u64 a = q < first ? p : nv - 1 - p;
+    const u64 b = q < first ? p + q : a + (q - first);
+    return vals[a] + vals[b];
+  }
+  // The key's slice, or ~0 when this build or pass does not take it.
+  __device__ __forceinline__ u32 slice(u64 k) const {
+    if (shards > 1 && fast_mod(mix64(k + kShardSeed), shards, srecip) != shard) return ~0u;
+    const u32 s = (u32)mulhi64(mix64(k), S);
+    return s >= s_lo && s < s_hi ? s : ~0u;
+  }
+  static constexpr int kItems = 1;   // items per element
+  __device__ __forceinline__ void get(u64 t, u64 (&item)[1], u32 (&sl)[1]) const {
+    item[0] = key(t);
+    sl[0] = slice(item[0]);
+  }
+};
+
+template <class Src>
+__global__ void __launch_bounds__(kPartThreads) k_part_count(Src src, u64 k0, u64 per, u64 k1, u32 S,
+                                                             u32* __restrict__ bhist) {
+  extern __shared__ u32 hist[];
+  for (u32 i = threadIdx.x; i < S; i += blockDim.x) hist[i] = 0;
+  __syncthreads();
+  const u64 lo = k0 + blockIdx.x * per, hi = min(k1, lo + per);
+  for (u64 t = lo + threadIdx.x; t < hi; t += blockDim.x) {
+    u64 item[Src::kItems];
+    u32 sl[Src::kItems];
+    src.get(t, item, sl);
+#pragma unroll
+    for (int j = 0; j < Src::kItems; ++j)
+      if (sl[j] != ~0u && S615_CHECK(sl[j] < S, kChkList)) atomicAdd(&hist[sl[j]], 1u);
+  }
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < S; i += blockDim.x) bhist[(u64)blockIdx.x * S + i] = hist[i];
+}
+
+// One block per slice: the exclusive scan of its G block counts, and its total.
+__global__ void k_part_scan(const u32* __restrict__ bhist, u32 G, u32 S,
+                            unsigned long long* __restrict__ brel,
+                            unsigned long long* __restrict__ total) {
+  __shared__ unsigned long long s_w[32];
+  const u32 sl = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long run = 0;
+  for (u32 b0 = 0; b0 < G; b0 += blockDim.x) {
+    const u32 b = b0 + threadIdx.x;
+    const unsigned long long c = b < G ? bhist[(u64)b * S + sl] : 0ull;
+    unsigned long long x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (u32)o) x += y;
+    }
+    if (lane == 31) s_w[wid] = x;
+    __syncthreads();
+    unsigned long long before = run, all = run;
+    for (u32 w = 0; w < blockDim.x / 32; ++w) {
+      if (w < wid) before += s_w[w];
+      all += s_w[w];
+    }
+    if (b < G) brel[(u64)b * S + sl] = before + x - c;
+    run = all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) total[sl] = run;
+}
+
+// soff[s] = items of slices [s0, s) for s in [s0, s1]; one block.
+__global__ void k_part_offsets(const unsigned long long* __restrict__ total, u32 s0, u32 s1,
+                               unsigned long long* __restrict__ soff) {
+  __shared__ unsigned long long s_w[32];
+  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long run = 0;
+  for (u32 b0 = s0; b0 < s1; b0 += blockDim.x) {
+    const u32 b = b0 + threadIdx.x;
+    const unsigned long long c = b < s1 ? total[b] : 0ull;
+    unsigned long long x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (u32)o) x += y;
+    }
+    if (lane == 31) s_w[wid] = x;
+    __syncthreads();
+    unsigned long long before = run, all = run;
+    for (u32 w = 0; w < blockDim.x / 32; ++w) {
+      if (w < wid) before += s_w[w];
+      all += s_w[w];
+    }
+    if (b < s1) soff[b] = before + x - c;
+    run = all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) soff[s1] = run;
+}
+
+// Dynamic shared memory of k_part_scatter: the staged tile, each staged item's
+// slice, and per slice its count, its start in the tile and its output cursor.
+constexpr size_t part_smem(u32 S) {
+  return (size_t)kTile * 8 + (size_t)S * 8 + (size_t)S * 4 * 2 + (size_t)kTile * 2;
+}
+
+template <class Src>
+__global__ void __launch_bounds__(kPartThreads, 2) k_part_scatter(
+    Src src, u64 k0, u64 per, u64 k1, u32 S, const unsigned long long* __restrict__ brel,
+    const unsigned long long* __restrict__ soff, unsigned long long* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned long long* stage = reinterpret_cast<unsigned long long*>(smem);
+  unsigned long long* cur = stage + kTile;
+  u32* cnt = reinterpret_cast<u32*>(cur + S);
+  u32* off = cnt + S;
+  u16* sid = reinterpret_cast<u16*>(off + S);
+  __shared__ u32 s_w[kPartThreads / 32];
+  constexpr int E = kPartPer / Src::kItems;   // elements per thread and tile
+  constexpr int I = E * Src::kItems;          // items per thread and tile (<= kPartPer)
+  const u32 tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (u32 i = tid; i < S; i += kPartThreads) {
+    cur[i] = soff[i] + brel[(u64)blockIdx.x * S + i];
+    cnt[i] = 0;
+  }
+  __syncthreads();
+  const u64 lo = k0 + blockIdx.x * per, hi = min(k1, lo + per);
+  for (u64 t0 = lo; t0 < hi; t0 += (u64)kPartThreads * E) {
+    u64 item[I];
+    u32 at[I];   // slice | rank in the tile's run << 13 (both below 2^13), ~0: none
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const u64 t = t0 + (u64)e * kPartThreads + tid;
+      u64 it[Src::kItems];
+      u32 sl[Src::kItems];
+#pragma unroll
+      for (int j = 0; j < Src::kItems; ++j) { it[j] = 0; sl[j] = ~0u; }
+      if (t < hi) src.get(t, it, sl);
+#pragma unroll
+      for (int j = 0; j < Src::kItems; ++j) {
+        const bool ok = sl[j] != ~0u && S615_CHECK(sl[j] < S, kChkList);
+        item[e * Src::kItems + j] = it[j];
+        at[e * Src::kItems + j] = ok ? sl[j] | (atomicAdd(&cnt[sl[j]], 1u) << 13) : ~0u;
+      }
+    }
+    __syncthreads();
+    // exclusive scan of the counts over the slices, ceil(S / threads) per thread
+    const u32 each = (S + kPartThreads - 1) / kPartThreads;
+    const u32 i0 = min(tid * each, S), i1 = min(i0 + each, S);
+    u32 sum = 0;
+    for (u32 i = i0; i < i1; ++i) sum += cnt[i];
+    u32 x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (u32)o) x += y;
+    }
+    if (lane == 31) s_w[wid] = x;
+    __syncthreads();
+    u32 before = 0, total = 0;
+    for (u32 w = 0; w < kPartThreads / 32; ++w) {
+      if (w < wid) before += s_w[w];
+      total += s_w[w];
+    }
+    u32 run = before + x - sum;
+    for (u32 i = i0; i < i1; ++i) { off[i] = run; run += cnt[i]; }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < I; ++k)
+      if (at[k] != ~0u) {
+        const u32 sl = at[k] & 8191u, pos = off[sl] + (at[k] >> 13);
+        stage[pos] = item[k];
+        sid[pos] = (u16)sl;
+      }
+    __syncthreads();
+    for (u32 pos = tid; pos < total; pos += kPartThreads) {
+      const u32 sl = sid[pos];
+      out[cur[sl] + (pos - off[sl])] = stage[pos];
+    }
+    __syncthreads();
+    for (u32 i = i0; i < i1; ++i) { cur[i] += cnt[i]; cnt[i] = 0; }
+    __syncthreads();
+  }
+}
+
+// One slice's keys into a hash set that stays in L2: a key is appended to out
+// when its insertion finds it new.  The other table is cleared meanwhile for
+// the next slice.  Four keys a thread, their probes in flight together.  A
+// full table (it has at least two slots a key) and the all-ones key set flags.
+// Bound by the round trips of the probes: 34 ms for the 1.15e9 keys of N =
+// 48,000 (46 ms with each key probed to its end in turn); a hash set of all keys
+// in HBM, scanned afterwards, took 110 ms or more.
+constexpr int kDedupPer = 4;
+static_assert(kDedupPer == 4, "the probe loop's condition");
+__global__ void k_dedupe(const u64* __restrict__ keys, u64 n, unsigned long long* table, u64 tmask,
+                         ulonglong2* clear, u64* __restrict__ out, u64 cap,
+                         unsigned long long* n_out, u32* flags) {
+  const u64 nt = (u64)gridDim.x * blockDim.x;
+  for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < (tmask + 1) / 2; i += nt)
+    clear[i] = make_ulonglong2(kEmpty, kEmpty);
+  const u64 span = (u64)blockDim.x * kDedupPer;
+  for (u64 base = blockIdx.x * span; base < n; base += (u64)gridDim.x * span) {
+    u64 key[kDedupPer], at[kDedupPer], old[kDedupPer];
+    bool fresh[kDedupPer], live[kDedupPer];
+#pragma unroll
+    for (int k = 0; k < kDedupPer; ++k) {
+      const u64 i = base + (u64)k * blockDim.x + threadIdx.x;
+      live[k] = i < n;
+      key[k] = live[k] ? keys[i] : 0;
+      if (live[k] && key[k] == kEmpty) { flags[0] = 1; live[k] = false; }
+      at[k] = mix64(key[k] ^ 0x5bd1e9955bd1e995ULL) & tmask;
+    }
+    // one probe of every unsettled key per step, so that a step is one round trip
+    // to L2 for the thread's keys together
+#pragma unroll
+    for (int k = 0; k < kDedupPer; ++k) fresh[k] = false;
+    for (u64 probe = 0; live[0] || live[1] || live[2] || live[3]; ++probe) {
+      if (probe > tmask) { flags[1] = 1; break; }
+#pragma unroll
+      for (int k = 0; k < kDedupPer; ++k)
+        if (live[k])
+          old[k] = atomicCAS(table + ((at[k] + probe) & tmask), (unsigned long long)kEmpty,
+                             (unsigned long long)key[k]);
+#pragma unroll
+      for (int k = 0; k < kDedupPer; ++k)
+        if (live[k]) {
+          fresh[k] = old[k] == kEmpty;
+          live[k] = !fresh[k] && old[k] != key[k];
+        }
+    }
+    u64 pos[kDedupPer];
+    block_positions<kDedupPer>(fresh, n_out, pos);   // every thread of the block, every pass
+#pragma unroll
+    for (int k = 0; k < kDedupPer; ++k)
+      if (fresh[k] && pos[k] < cap) out[pos[k]] = key[k];   // past cap: counted, not written
   }
 }
 
@@ -201,53 +434,27 @@ __global__ void k_max_count(const unsigned long long* __restrict__ W, u64 m, uns
 
 // ---- incidence through shared-memory radix bins ---------------------------
 // The cells are cut into slices of 2^sbits cells (16 MB of cell words:
-// L2-sized).  Each block takes a fixed range of keys.  k_bin_count counts the
-// block's updates per slice in a shared-memory histogram; a host scan over
-// (slice, block) gives every block its own output range per slice;
-// k_bin_scatter bins the updates through shared-memory cursors into those
-// ranges (slice-local cell offset and key index, 8 B), so the updates of a
-// slice lie together; k_bin_apply walks them slice by slice with the whole
-// grid, and its atomic adds land on a slice that is resident in L2.
-constexpr u32 kMaxSlices = 4608;
-constexpr int kBinThreads = 256;
-
-__global__ void k_bin_count(const u64* __restrict__ keys, u64 k0, u64 per, u64 k1, u64 seed,
-                            u64 block, u64 recip, u32 sbits, u32 S, u32* __restrict__ bhist) {
-  extern __shared__ u32 hist[];
-  for (u32 i = threadIdx.x; i < S; i += blockDim.x) hist[i] = 0;
-  __syncthreads();
-  const u64 lo = k0 + blockIdx.x * per, hi = min(k1, lo + per);
-  for (u64 i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+// L2-sized) and the three updates of every key are partitioned by slice (one
+// 8-byte entry each: key index << 32 | slice-local cell offset); k_bin_apply
+// walks them slice by slice with the whole grid, and its atomic adds land on a
+// slice that is resident in L2.
+struct UpdateSource {
+  const u64* keys;
+  u64 k0, seed, block, recip;
+  u32 sbits;
+  static constexpr int kItems = 3;
+  __device__ __forceinline__ void get(u64 i, u64 (&item)[3], u32 (&sl)[3]) const {
     u64 c[3];
     cell_indices(key_hash(keys, i, seed), block, recip, c);
-    if (!cells_ok(c, block) || !S615_CHECK(((3 * block - 1) >> sbits) < S, kChkList)) continue;
-#pragma unroll
-    for (int t = 0; t < 3; ++t) atomicAdd(&hist[(u32)(c[t] >> sbits)], 1u);
-  }
-  __syncthreads();
-  for (u32 i = threadIdx.x; i < S; i += blockDim.x) bhist[(u64)blockIdx.x * S + i] = hist[i];
-}
-
-__global__ void k_bin_scatter(const u64* __restrict__ keys, u64 k0, u64 per, u64 k1, u64 seed,
-                              u64 block, u64 recip, u32 sbits, u32 S,
-                              const unsigned long long* __restrict__ bbase,
-                              unsigned long long* __restrict__ ent) {
-  extern __shared__ unsigned long long cur[];
-  for (u32 i = threadIdx.x; i < S; i += blockDim.x) cur[i] = bbase[(u64)blockIdx.x * S + i];
-  __syncthreads();
-  const u64 lo = k0 + blockIdx.x * per, hi = min(k1, lo + per);
-  const u64 lmask = (1ull << sbits) - 1;
-  for (u64 i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    u64 c[3];
-    cell_indices(key_hash(keys, i, seed), block, recip, c);
-    if (!cells_ok(c, block) || !S615_CHECK(((3 * block - 1) >> sbits) < S, kChkList)) continue;
+    const bool ok = cells_ok(c, block);
+    const u64 lmask = (1ull << sbits) - 1;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-      const unsigned long long pos = atomicAdd(&cur[(u32)(c[t] >> sbits)], 1ull);
-      ent[pos] = ((u64)(i - k0) << 32) | (c[t] & lmask);   // one 8-byte store per update
+      item[t] = ((i - k0) << 32) | (c[t] & lmask);
+      sl[t] = ok ? (u32)(c[t] >> sbits) : ~0u;
     }
   }
-}
+};
 
 // A cooperative grid walks the slices in order and splits each slice's
 // entries over all its threads, with a grid-wide sync after every slice, so
@@ -298,57 +505,16 @@ struct CellList {
   __device__ __forceinline__ u64 cell(u64 k, u64 block) const { return third[k] * block + off[k]; }
 };
 
-// Append up to two flagged cells per thread with ONE global atomic per block:
-// each warp's count goes to shared memory, thread 0 reserves the block's
-// total, and every lane writes at its offset.  All appends of a list go
-// through one counter, so per-warp atomics on it serialise in its L2 slice:
-// at ~1.7e8 such atomics/s they bound the round's apply (ncu: DRAM 11%, L2 5%,
-// 578 long-scoreboard stall cycles per issue); per block they are 8x fewer.
-// Every thread of the block calls this (it synchronises the block); it
-// returns the first entry's position, or ~0 when not taken or over capacity.
-__device__ __forceinline__ u64 block_append(bool take0, u64 c0, bool take1, u64 c1, u64 block,
-                                            CellList list, unsigned long long* count, u64 cap,
-                                            u32* over) {
-  __shared__ u32 s_cnt[32];
-  __shared__ unsigned long long s_base;
-  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  const u32 b0 = __ballot_sync(0xFFFFFFFFu, take0), b1 = __ballot_sync(0xFFFFFFFFu, take1);
-  __syncthreads();   // the previous call's offsets have been read
-  if (lane == 0) s_cnt[wid] = __popc(b0) + __popc(b1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    u32 tot = 0;
-    for (u32 w = 0; w < nw; ++w) {
-      const u32 k = s_cnt[w];
-      s_cnt[w] = tot;
-      tot += k;
-    }
-    s_base = tot ? atomicAdd(count, (unsigned long long)tot) : 0ull;
+// Write cell c at position `at` of the list, or set *over past its capacity.
+__device__ __forceinline__ bool list_put(CellList list, u64 at, u64 cap, u64 c, u64 block, u32* over) {
+  if (at >= cap) {
+    *over = 1;
+    return false;
   }
-  __syncthreads();
-  const u64 at0 = s_base + s_cnt[wid] + __popc(b0 & ((1u << lane) - 1u));
-  const u64 at1 = s_base + s_cnt[wid] + __popc(b0) + __popc(b1 & ((1u << lane) - 1u));
-  u64 first = ~0ull;
-  if (take0) {
-    if (at0 < cap) {
-      const u32 t = c0 >= 2 * block ? 2u : c0 >= block ? 1u : 0u;
-      list.off[at0] = (u32)(c0 - t * block);
-      list.third[at0] = (u8)t;
-      first = at0;
-    } else {
-      *over = 1;
-    }
-  }
-  if (take1) {
-    if (at1 < cap) {
-      const u32 t = c1 >= 2 * block ? 2u : c1 >= block ? 1u : 0u;
-      list.off[at1] = (u32)(c1 - t * block);
-      list.third[at1] = (u8)t;
-    } else {
-      *over = 1;
-    }
-  }
-  return first;
+  const u32 t = c >= 2 * block ? 2u : c >= block ? 1u : 0u;
+  list.off[at] = (u32)(c - t * block);
+  list.third[at] = (u8)t;
+  return true;
 }
 
 // The claimed cells of the peel, in round order.  With idx and hash set
@@ -364,40 +530,56 @@ struct ClaimList {
   }
 };
 
-// Does cell c (count 1) claim its key?  The key's lower count-1 cells win.
-__device__ __forceinline__ bool claims(const unsigned long long* W, const u64* keys, u64 seed,
-                                       u64 block, u64 recip, u64 c, u64 w, u64& h) {
-  h = key_hash(keys, w & kSumMask, seed);
-  u64 cs[3];
-  cell_indices(h, block, recip, cs);
-  if (!cells_ok(cs, block)) return false;
-#pragma unroll
-  for (int t = 0; t < 3; ++t)
-    if (cs[t] < c && cnt_of(W[cs[t]]) == 1) return false;
-  return true;
-}
-
 // Claims among the candidate cells [0, ncand), or among every cell when the
-// candidate list is null.
+// candidate list is null: a count-1 cell claims its key unless a lower cell of
+// the key has count 1 too.  A candidate costs a chain of scattered reads (its
+// word, its key, the key's lower cells), so each thread follows kClaimPer
+// chains at once.
+constexpr int kClaimPer = 4;
 __global__ void k_claim_list(CellList cand, u64 ncand, const unsigned long long* __restrict__ W,
                              const u64* __restrict__ keys, u64 seed, u64 block, u64 recip,
                              ClaimList out, unsigned long long* n_order, u64 order_cap, u32* over) {
-  for (u64 base = blockIdx.x * (u64)blockDim.x; base < ncand; base += (u64)gridDim.x * blockDim.x) {
-    const u64 i = base + threadIdx.x;
-    bool claim = false;
-    u64 c = 0, w = 0, h = 0;
-    if (i < ncand) {
-      c = cand.off ? cand.cell(i, block) : i;
-      if (S615_CHECK(c < 3 * block, kChkList)) {
-        w = W[c];
-        claim = cnt_of(w) == 1 && claims(W, keys, seed, block, recip, c, w, h);
+  const u64 span = (u64)blockDim.x * kClaimPer;
+  for (u64 base = blockIdx.x * span; base < ncand; base += (u64)gridDim.x * span) {
+    bool claim[kClaimPer];
+    u64 c[kClaimPer], w[kClaimPer], h[kClaimPer];
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k) {
+      const u64 i = base + (u64)k * blockDim.x + threadIdx.x;
+      claim[k] = i < ncand;
+      c[k] = claim[k] ? (cand.off ? cand.cell(i, block) : i) : 0;
+      claim[k] = claim[k] && S615_CHECK(c[k] < 3 * block, kChkList);
+    }
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k) w[k] = claim[k] ? W[c[k]] : 0;
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k) {
+      claim[k] = claim[k] && cnt_of(w[k]) == 1;
+      h[k] = claim[k] ? key_hash(keys, w[k] & kSumMask, seed) : 0;
+    }
+    u64 w0[kClaimPer], w1[kClaimPer];   // the words of the key's lower cells, 0: none
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k) {
+      w0[k] = w1[k] = 0;
+      if (claim[k]) {
+        u64 cs[3];
+        cell_indices(h[k], block, recip, cs);
+        claim[k] = cells_ok(cs, block);
+        if (claim[k] && cs[0] < c[k]) w0[k] = W[cs[0]];
+        if (claim[k] && cs[1] < c[k]) w1[k] = W[cs[1]];
       }
     }
-    const u64 k = block_append(claim, c, false, 0, block, out.cells, n_order, order_cap, over);
-    if (k != ~0ull && out.hash) {
-      out.idx[k] = (u32)(w & kSumMask);
-      out.hash[k] = h;
-    }
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k)
+      claim[k] = claim[k] && cnt_of(w0[k]) != 1 && cnt_of(w1[k]) != 1;
+    u64 pos[kClaimPer];
+    block_positions<kClaimPer>(claim, n_order, pos);   // every thread of the block, every pass
+#pragma unroll
+    for (int k = 0; k < kClaimPer; ++k)
+      if (claim[k] && list_put(out.cells, pos[k], order_cap, c[k], block, over) && out.hash) {
+        out.idx[pos[k]] = (u32)(w[k] & kSumMask);
+        out.hash[pos[k]] = h[k];
+      }
   }
 }
 
@@ -405,53 +587,6 @@ __global__ void k_claim_list(CellList cand, u64 ncand, const unsigned long long*
 // are in flight together, and the block synchronises (in the append) once
 // per pass instead of once per key.
 constexpr int kApplyPer = 4;
-
-// block_append for K cells per thread (flags take[k], cells c[k]), one global
-// atomic per block; every thread of the block calls it.
-template <int K>
-__device__ __forceinline__ void block_append_n(const bool (&take)[K], const u64 (&c)[K], u64 block,
-                                               CellList list, unsigned long long* count, u64 cap,
-                                               u32* over) {
-  __shared__ u32 s_cnt[32];
-  __shared__ unsigned long long s_base;
-  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  u32 b[K];
-  u32 wtot = 0;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    b[k] = __ballot_sync(0xFFFFFFFFu, take[k]);
-    wtot += __popc(b[k]);
-  }
-  __syncthreads();   // the previous call's offsets have been read
-  if (lane == 0) s_cnt[wid] = wtot;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    u32 tot = 0;
-    for (u32 w = 0; w < nw; ++w) {
-      const u32 n = s_cnt[w];
-      s_cnt[w] = tot;
-      tot += n;
-    }
-    s_base = tot ? atomicAdd(count, (unsigned long long)tot) : 0ull;
-  }
-  __syncthreads();
-  u64 at = s_base + s_cnt[wid];
-  const u32 below = (1u << lane) - 1u;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (take[k]) {
-      const u64 pos = at + __popc(b[k] & below);
-      if (pos < cap) {
-        const u32 t = c[k] >= 2 * block ? 2u : c[k] >= block ? 1u : 0u;
-        list.off[pos] = (u32)(c[k] - t * block);
-        list.third[pos] = (u8)t;
-      } else {
-        *over = 1;
-      }
-    }
-    at += __popc(b[k]);
-  }
-}
 
 __global__ void k_apply_list(ClaimList in, u64 L, unsigned long long* W,
                              const u64* __restrict__ keys, u64 seed, u64 block, u64 recip,
@@ -483,13 +618,17 @@ __global__ void k_apply_list(ClaimList in, u64 L, unsigned long long* W,
         cell_indices(h, block, recip, cs);
         if (cells_ok(cs, block) && S615_KEY_OK(idx)) {   // always true in the default build
           const int own = cs[0] == c ? 0 : cs[1] == c ? 1 : 2;
-          nc[2 * q] = cs[own == 0 ? 1 : 0];
-          nc[2 * q + 1] = cs[own == 2 ? 1 : 2];
+          nc[2 * q] = own == 0 ? cs[1] : cs[0];
+          nc[2 * q + 1] = own == 2 ? cs[1] : cs[2];
           old[2 * q] = atomicAdd(W + nc[2 * q], (unsigned long long)(0 - upd(idx)));
           old[2 * q + 1] = atomicAdd(W + nc[2 * q + 1], (unsigned long long)(0 - upd(idx)));
           to[2 * q] = to[2 * q + 1] = true;   // pending: the count check follows
-          // count 0; without the recorded index the word keeps it for the fill
-          W[c] = in.hash ? 0ull : idx;
+          // Without the recorded index the word keeps it, at count 0, for the
+          // fill.  With it the word is left as it is (count 1): no unpeeled key
+          // has this cell, so nothing but a scan of every cell would read it
+          // again before the fill writes it (k_zero_claimed goes before such a
+          // scan).  The store would be a third scattered update per key.
+          if (!in.hash) W[c] = idx;
         }
       }
     }
@@ -497,7 +636,11 @@ __global__ void k_apply_list(ClaimList in, u64 L, unsigned long long* W,
 #pragma unroll
     for (int k = 0; k < 2 * kApplyPer; ++k) to[k] = to[k] && cnt_of(old[k]) == 2;
     // every thread of the block reaches the append (it synchronises the block)
-    block_append_n<2 * kApplyPer>(to, nc, block, next, n_next, next_cap, over);
+    u64 pos[2 * kApplyPer];
+    block_positions<2 * kApplyPer>(to, n_next, pos);
+#pragma unroll
+    for (int k = 0; k < 2 * kApplyPer; ++k)
+      if (to[k]) list_put(next, pos[k], next_cap, nc[k], block, over);
   }
 }
 
@@ -516,13 +659,47 @@ __device__ __forceinline__ void fill_cell(unsigned long long* W, u64 h, u64 bloc
   W[c] = v & mask;
 }
 
+// Count 0 for the claimed cells, before a round that scans every cell.
+__global__ void k_zero_claimed(CellList in, u64 L, unsigned long long* W, u64 block) {
+  const u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x;
+  if (i < L && S615_CHECK(in.cell(i, block) < 3 * block, kChkList)) W[in.cell(i, block)] = 0ull;
+}
+
+constexpr int kFillPer = 4;   // fills in flight per thread
 __global__ void k_fill_list(ClaimList in, u64 L, unsigned long long* W,
                             const u64* __restrict__ keys, u64 seed, u64 block, u64 recip, u64 mask) {
-  for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < L;
-       i += (u64)gridDim.x * blockDim.x) {
-    const u64 c = in.cells.cell(i, block);
-    const u64 h = in.hash ? (u64)in.hash[i] : key_hash(keys, W[c], seed);
-    fill_cell(W, h, block, recip, mask, c);
+  const u64 span = (u64)blockDim.x * kFillPer;
+  for (u64 base = blockIdx.x * span; base < L; base += (u64)gridDim.x * span) {
+    u64 c[kFillPer], h[kFillPer], v[kFillPer];
+    bool on[kFillPer];
+#pragma unroll
+    for (int k = 0; k < kFillPer; ++k) {
+      const u64 i = base + (u64)k * blockDim.x + threadIdx.x;
+      on[k] = i < L;
+      c[k] = on[k] ? in.cells.cell(i, block) : 0;
+      on[k] = on[k] && S615_CHECK(c[k] < 3 * block, kChkList);
+      h[k] = on[k] && in.hash ? (u64)in.hash[i] : 0;
+    }
+    if (!in.hash) {
+#pragma unroll
+      for (int k = 0; k < kFillPer; ++k) h[k] = on[k] ? key_hash(keys, W[c[k]], seed) : 0;
+    }
+    // the key's other two cells: claimed in a later round or never, so no
+    // thread of this launch writes them
+#pragma unroll
+    for (int k = 0; k < kFillPer; ++k) {
+      v[k] = 0;
+      if (on[k]) {
+        u64 cs[3];
+        cell_indices(h[k], block, recip, cs);
+        on[k] = cells_ok(cs, block);
+        const int own = cs[0] == c[k] ? 0 : cs[1] == c[k] ? 1 : 2;
+        if (on[k]) v[k] = W[own == 0 ? cs[1] : cs[0]] ^ W[own == 2 ? cs[1] : cs[2]];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kFillPer; ++k)
+      if (on[k]) W[c[k]] = (v[k] ^ h[k]) & mask;
   }
 }
 
@@ -539,6 +716,18 @@ __device__ __forceinline__ void remove_key_scan(unsigned long long* W, const u64
   W[c] = idx;   // count 0; the index stays for the fill
 }
 
+// Does cell c (count 1) claim its key?  The key's lower count-1 cells win.
+__device__ __forceinline__ bool claims(const unsigned long long* W, const u64* keys, u64 seed,
+                                       u64 block, u64 recip, u64 c, u64 w) {
+  u64 cs[3];
+  cell_indices(key_hash(keys, w & kSumMask, seed), block, recip, cs);
+  if (!cells_ok(cs, block)) return false;
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+    if (cs[t] < c && cnt_of(W[cs[t]]) == 1) return false;
+  return true;
+}
+
 // The scan form: claims of round r tagged in round[], apply and fill by tag.
 __global__ void k_claim_scan(const unsigned long long* __restrict__ W, const u64* __restrict__ keys,
                              u64 seed, u16* __restrict__ round, u64 m, u64 block, u64 recip, u16 r,
@@ -548,11 +737,12 @@ __global__ void k_claim_scan(const unsigned long long* __restrict__ W, const u64
     bool claim = false;
     if (c < m) {
       const u64 w = W[c];
-      u64 h;
-      claim = cnt_of(w) == 1 && claims(W, keys, seed, block, recip, c, w, h);
+      claim = cnt_of(w) == 1 && claims(W, keys, seed, block, recip, c, w);
       if (claim) round[c] = r;
     }
-    block_reserve(claim, n_claimed);   // counts the claims (every thread, every pass)
+    const bool take[1] = {claim};
+    u64 pos[1];
+    block_positions<1>(take, n_claimed, pos);   // counts the claims (every thread, every pass)
   }
 }
 
@@ -588,55 +778,73 @@ struct Buf {
   ~Buf() { release(); }
 };
 
-u64 pow2_at_least(u64 x) { u64 p = 1; while (p < x) p <<= 1; return p; }
+// The scratch of a partition into at most S slices by G blocks: per-block
+// counts and bases, slice totals and offsets.
+struct PartScratch {
+  u32* bhist;
+  unsigned long long *brel, *total, *soff;
+  static size_t bytes(size_t G, size_t S) { return G * S * 12 + (2 * S + 1) * 8 + 64; }
+  PartScratch(void* p, size_t G, size_t S) {
+    brel = static_cast<unsigned long long*>(p);
+    total = brel + G * S;
+    soff = total + S;
+    bhist = reinterpret_cast<u32*>(soff + S + 1);
+  }
+};
+
+// Count: the items of elements [k0, k1) per slice, in ps.total and ps.brel.
+template <class Src>
+int part_count(s615_ctx* ctx, const Src& src, u64 k0, u64 k1, u32 G, u32 S, const PartScratch& ps,
+               cudaStream_t st) {
+  k_part_count<Src><<<G, kPartThreads, S * sizeof(u32), st>>>(src, k0, (k1 - k0 + G - 1) / G, k1, S, ps.bhist);
+  k_part_scan<<<S, 256, 0, st>>>(ps.bhist, G, S, ps.brel, ps.total);
+  ctx->launches += 2;
+  S615_CU(cudaGetLastError());
+  return S615_OK;
+}
+
+// Scatter the items of slices [s0, s1) (counted by part_count over the same
+// elements) to out, slice after slice; ps.soff[s0 .. s1] are their offsets.
+template <class Src>
+int part_scatter(s615_ctx* ctx, const Src& src, u64 k0, u64 k1, u32 G, u32 S, u32 s0, u32 s1,
+                 const PartScratch& ps, unsigned long long* out, cudaStream_t st) {
+  S615_CU(cudaFuncSetAttribute(k_part_scatter<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)part_smem(kMaxSlices)));
+  k_part_offsets<<<1, 1024, 0, st>>>(ps.total, s0, s1, ps.soff);
+  k_part_scatter<Src><<<G, kPartThreads, part_smem(S), st>>>(src, k0, (k1 - k0 + G - 1) / G, k1, S,
+                                                             ps.brel, ps.soff, out);
+  ctx->launches += 2;
+  S615_CU(cudaGetLastError());
+  return S615_OK;
+}
+
+// Blocks of a partition pass: two per SM, fewer for few elements.
+u32 part_blocks(const s615_ctx* ctx, u64 n) {
+  return (u32)std::min<u64>((u64)ctx->num_sms * 2, std::max<u64>(1, n / (4 * kTile)));
+}
 
 // Incidence of keys [0, n) for one seed through the slice bins, in chunks of
 // keys whose updates fit the entry buffers (ent_cap updates).
 int incidence_binned(s615_ctx* ctx, const u64* keys, u64 n, u64 seed, u64 m, u64 block, u64 recip,
-                     unsigned long long* ent, u64 ent_cap, unsigned long long* W, u32* bhist,
-                     unsigned long long* bbase, cudaStream_t st) {
+                     unsigned long long* ent, u64 ent_cap, unsigned long long* W, void* scratch,
+                     cudaStream_t st) {
   u32 sbits = 21;
   while (((m + (1ull << sbits) - 1) >> sbits) > kMaxSlices) ++sbits;
   const u32 S = (u32)((m + (1ull << sbits) - 1) >> sbits);
-  const int G = ctx->num_sms * 2;
   const u64 chunk = std::max<u64>(1, std::min<u64>(ent_cap / 3, 1ull << 32));
-  std::vector<u32> h_hist((size_t)G * S);
-  std::vector<unsigned long long> h_base((size_t)G * S), h_soff(S + 1);
   for (u64 k0 = 0; k0 < n; k0 += chunk) {
     const u64 k1 = std::min(n, k0 + chunk);
-    const u64 per = (k1 - k0 + G - 1) / G;
-    k_bin_count<<<G, kBinThreads, S * sizeof(u32), st>>>(keys, k0, per, k1, seed, block, recip, sbits,
-                                                         S, bhist);
-    ctx->launches++;
-    S615_CU(cudaGetLastError());
-    S615_CU(cudaMemcpyAsync(h_hist.data(), bhist, h_hist.size() * sizeof(u32), cudaMemcpyDeviceToHost, st));
-    S615_CU(cudaStreamSynchronize(st));
-    // exclusive scan in (slice, block) order: slice s's updates are contiguous
-    unsigned long long run = 0;
-    for (u32 sl = 0; sl < S; ++sl) {
-      h_soff[sl] = run;
-      for (int b = 0; b < G; ++b) {
-        h_base[(size_t)b * S + sl] = run;
-        run += h_hist[(size_t)b * S + sl];
-      }
-    }
-    h_soff[S] = run;
-    if (run != 3 * (k1 - k0)) return S615_E_DEVICE;
-    S615_CU(cudaMemcpyAsync(bbase, h_base.data(), h_base.size() * sizeof(unsigned long long),
-                            cudaMemcpyHostToDevice, st));
-    k_bin_scatter<<<G, kBinThreads, S * sizeof(unsigned long long), st>>>(
-        keys, k0, per, k1, seed, block, recip, sbits, S, bbase, ent);
-    ctx->launches++;
-    S615_CU(cudaGetLastError());
-    // the slice starts go where the block bases were (read by the apply kernel)
-    S615_CU(cudaMemcpyAsync(bbase, h_soff.data(), (S + 1) * sizeof(unsigned long long),
-                            cudaMemcpyHostToDevice, st));
+    const u32 G = part_blocks(ctx, k1 - k0);
+    const PartScratch ps(scratch, G, S);
+    const UpdateSource src{keys, k0, seed, block, recip, sbits};
+    if (const int s = part_count(ctx, src, k0, k1, G, S, ps, st)) return s;
+    if (const int s = part_scatter(ctx, src, k0, k1, G, S, 0, S, ps, ent, st)) return s;
     int per_sm = 0;
     S615_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bin_apply<true>, 256, 0));
     const dim3 grid(ctx->num_sms * std::max(per_sm, 1));
     {   // cooperative: every block resident at once (the launch is refused otherwise)
       const unsigned long long* a_ent = ent;
-      const unsigned long long* a_soff = bbase;
+      const unsigned long long* a_soff = ps.soff;
       u64 a_k0 = k0;
       u32 a_sbits = sbits, a_S = S;
       void* args[] = {(void*)&a_ent, (void*)&a_k0, (void*)&a_soff, (void*)&a_sbits, (void*)&a_S,
@@ -644,12 +852,84 @@ int incidence_binned(s615_ctx* ctx, const u64* keys, u64 n, u64 seed, u64 m, u64
       if (cudaLaunchCooperativeKernel((const void*)k_bin_apply<true>, grid, dim3(256), args, 0, st) !=
           cudaSuccess) {
         cudaGetLastError();
-        k_bin_apply<false><<<grid, 256, 0, st>>>(ent, k0, bbase, sbits, S, W);
+        k_bin_apply<false><<<grid, 256, 0, st>>>(ent, k0, ps.soff, sbits, S, W);
       }
     }
     ctx->launches++;
     S615_CU(cudaGetLastError());
-    S615_CU(cudaStreamSynchronize(st));   // h_base / h_soff are reused by the next chunk
+  }
+  return S615_OK;
+}
+
+// The distinct keys of src (at most cap) to out; *n their number.  Slices of
+// about 1.5 million keys, so that a slice's hash set (32 MB, and the next one's
+// being cleared) stays in L2; more and smaller ones when HBM is short, and
+// then as many passes over the source as the partition buffer needs.
+int unique_keys(s615_ctx* ctx, KeySource src, u64 n_raw, size_t avail, u64* out, u64 cap, u64* n,
+                cudaStream_t st) {
+  constexpr u64 kSliceKeys = 3ull << 19, kMost = 4096;
+  u64 S = std::min<u64>(kMost, (n_raw + kSliceKeys - 1) / kSliceKeys);
+  S = std::max<u64>(S, 1);
+  // two tables of up to four slots a key, in at most a quarter of the room
+  while (S < kMost && (n_raw / S + 1) * 8 * 8 > avail / 4) S = std::min<u64>(kMost, 2 * S);
+  const u32 G = part_blocks(ctx, src.n);
+  src.S = (u32)S;
+  src.s_lo = 0;
+  src.s_hi = (u32)S;
+  Buf scratch(ctx), part(ctx), tables(ctx);
+  int s = scratch.alloc(PartScratch::bytes(G, S) + 64);
+  if (s) return s;
+  auto* d_n = static_cast<unsigned long long*>(scratch.p);           // [0] count
+  u32* d_flags = reinterpret_cast<u32*>(d_n + 1);                    // all-ones key, full table
+  const PartScratch ps(static_cast<char*>(scratch.p) + 64, G, S);
+  S615_CU(cudaMemsetAsync(scratch.p, 0, 64, st));
+  if ((s = part_count(ctx, src, 0, src.n, G, (u32)S, ps, st))) return s;
+  std::vector<unsigned long long> total(S);
+  S615_CU(cudaMemcpyAsync(total.data(), ps.total, S * 8, cudaMemcpyDeviceToHost, st));
+  S615_CU(cudaStreamSynchronize(st));
+  u64 most = 0, all = 0;
+  for (u64 t : total) { most = std::max<u64>(most, t); all += t; }
+  u64 slots = 1024;
+  while (slots < 2 * most) slots *= 2;
+  if ((s = tables.alloc(2 * slots * 8))) return s;
+  auto* T = static_cast<unsigned long long*>(tables.p);
+  S615_CU(cudaMemsetAsync(T, 0xFF, 2 * slots * 8, st));
+  // the partition buffer: every key when there is room, else what there is
+  const size_t held = 2 * slots * 8 + PartScratch::bytes(G, S);
+  const u64 room = avail > held ? (avail - held) / 8 : 0;
+  const u64 part_cap = std::max<u64>(std::min<u64>(all, room), std::max<u64>(most, 1));
+  if ((s = part.alloc(part_cap * 8))) return s;
+  auto* P = static_cast<unsigned long long*>(part.p);
+  u32 flip = 0;
+  for (u32 s0 = 0; s0 < S;) {
+    u32 s1 = s0;
+    u64 held_keys = 0;
+    while (s1 < S && (s1 == s0 || held_keys + total[s1] <= part_cap)) held_keys += total[s1++];
+    src.s_lo = s0;
+    src.s_hi = s1;
+    if ((s = part_scatter(ctx, src, 0, src.n, G, (u32)S, s0, s1, ps, P, st))) return s;
+    u64 at = 0;
+    for (u32 sl = s0; sl < s1; ++sl) {
+      if (!total[sl]) continue;
+      k_dedupe<<<blocks_for(total[sl], 256 * kDedupPer), 256, 0, st>>>(
+          reinterpret_cast<const u64*>(P + at), total[sl], T + flip * slots, slots - 1,
+          reinterpret_cast<ulonglong2*>(T + (flip ^ 1) * slots), out, cap, d_n, d_flags);
+      ctx->launches++;
+      flip ^= 1;
+      at += total[sl];
+    }
+    S615_CU(cudaGetLastError());
+    s0 = s1;
+  }
+  unsigned long long h[2] = {0, 0};
+  S615_CU(cudaMemcpyAsync(h, d_n, 16, cudaMemcpyDeviceToHost, st));
+  S615_CU(cudaStreamSynchronize(st));
+  if (h[0] > cap || (h[1] >> 32)) return S615_E_BUILD;   // more keys than out holds, or a full table
+  *n = h[0];
+  if (h[1] & 0xFFFFFFFFull) {   // the all-ones key stays out of the hash set (out has room for it)
+    const u64 e = kEmpty;
+    S615_CU(cudaMemcpy(out + *n, &e, 8, cudaMemcpyHostToDevice));
+    ++*n;
   }
   return S615_OK;
 }
@@ -710,59 +990,21 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     // +1: the all-ones key is kept out of the hash set and appended last
     int s = keys.alloc((n_raw + 1) * sizeof(u64));
     if (s) return s;
-    // Hash set sized for load <= 1/2 per partition; partitions by the top bits
-    // of mix64(key) bound the table when HBM is short.
     release_run_batch(ctx);   // a table needs the room more than s615_run's kept buffers
     size_t free_b = 0, total_b = 0;
     S615_CU(cudaMemGetInfo(&free_b, &total_b));
     size_t avail = std::min(free_b, budget_room(ctx));
     if (avail > ((size_t)2 << 30)) avail -= (size_t)2 << 30;
-    u32 part_bits = 0;
-    u64 tsize = pow2_at_least(std::max<u64>(2 * n_raw, 1024));
-    while (tsize * sizeof(u64) > avail && part_bits < 8) {
-      ++part_bits;
-      tsize = pow2_at_least(std::max<u64>((2 * n_raw >> part_bits) + (n_raw >> (part_bits + 3)) + 1024, 1024));
-    }
-    Buf table(ctx), scratch(ctx);
-    s = table.alloc(tsize * sizeof(u64));
-    if (s) return s;
-    s = scratch.alloc(64);
-    if (s) return s;
-    u32* d_flag = static_cast<u32*>(scratch.p);
-    unsigned long long* d_n = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch.p) + 8);
-    S615_CU(cudaMemsetAsync(scratch.p, 0, 64, st));
-    for (u32 part = 0; part < (1u << part_bits); ++part) {
-      S615_CU(cudaMemsetAsync(table.p, 0xFF, tsize * sizeof(u64), st));
-      const KeyFilter kf{part_bits, part, shards, shard, mod_recip(shards)};
-      if (pairs) {
-        const int grid = (int)std::min<u64>(n_vals ? n_vals : 1, (u64)ctx->num_sms * 32);
-        k_insert_pairs<<<grid, 256, 0, st>>>(d_pair_vals, n_vals,
-                                             static_cast<unsigned long long*>(table.p), tsize - 1,
-                                             kf, d_flag);
-      } else {
-        k_insert_keys<<<grid_for(ctx, n_keys, 256), 256, 0, st>>>(
-            d_keys, n_keys, static_cast<unsigned long long*>(table.p), tsize - 1, kf, d_flag);
-      }
-      ctx->launches++;
-      S615_CU(cudaGetLastError());
-      k_compact<<<grid_for(ctx, tsize, 256), 256, 0, st>>>(
-          static_cast<const unsigned long long*>(table.p), tsize, static_cast<u64*>(keys.p), n_raw,
-          d_n);
-      ctx->launches++;
-      S615_CU(cudaGetLastError());
-    }
-    u32 h_flag = 0;
-    unsigned long long h_n = 0;
-    S615_CU(cudaMemcpyAsync(&h_flag, d_flag, 4, cudaMemcpyDeviceToHost, st));
-    S615_CU(cudaMemcpyAsync(&h_n, d_n, 8, cudaMemcpyDeviceToHost, st));
-    S615_CU(cudaStreamSynchronize(st));
-    n = h_n;
-    if (n > n_raw) return S615_E_BUILD;   // more keys in this shard than its buffer holds
-    if (h_flag) {
-      const u64 e = kEmpty;
-      S615_CU(cudaMemcpy(static_cast<u64*>(keys.p) + n, &e, 8, cudaMemcpyHostToDevice));
-      ++n;
-    }
+    KeySource src{};
+    src.vals = d_pair_vals;
+    src.keys = d_keys;
+    src.nv = n_vals;
+    src.n = n_all;
+    src.row_recip = mod_recip(n_vals + 1);
+    src.shards = shards;
+    src.shard = shard;
+    src.srecip = mod_recip(shards);
+    if ((s = unique_keys(ctx, src, n_raw, avail, static_cast<u64*>(keys.p), n_raw, &n, st))) return s;
   }
 
   std::memset(&out->hdr, 0, sizeof out->hdr);
@@ -820,7 +1062,7 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     const size_t margin = (size_t)2 << 30;
     return a > margin ? a - margin : 0;
   };
-  const size_t bin_bytes = (size_t)ctx->num_sms * 2 * kMaxSlices * (4 + 8) + 64;
+  const size_t bin_bytes = PartScratch::bytes((size_t)ctx->num_sms * 2, kMaxSlices);
   // the recorded claim list needs 17 bytes per key in the entry buffers
   // (offset, third, u32 index, hash) and n < 2^32; otherwise the claimed
   // cells alone (5 bytes per key) are taken now, before the entry buffers
@@ -876,13 +1118,8 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     if (!lists) S615_CU(cudaMemsetAsync(rounds.p, 0, m * sizeof(u16), st));
     S615_CU(cudaMemsetAsync(scratch.p, 0, 64, st));
     if (ent_cap) {
-      const size_t G = (size_t)ctx->num_sms * 2;
-      u32* bhist = static_cast<u32*>(bins.p);
-      auto* bbase = reinterpret_cast<unsigned long long*>(static_cast<char*>(bins.p) +
-                                                          (G * kMaxSlices * 4 + 7) / 8 * 8);
       if ((s = incidence_binned(ctx, K, n, seed, m, block, recip,
-                                static_cast<unsigned long long*>(ent.p), ent_cap, W, bhist, bbase,
-                                st)))
+                                static_cast<unsigned long long*>(ent.p), ent_cap, W, bins.p, st)))
         return s;
     } else {
       k_incidence<<<grid_for(ctx, n, 256), 256, 0, st>>>(K, n, seed, block, recip, W);
@@ -915,9 +1152,8 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
       std::vector<std::array<double, 4>> rounds_trace;
       while (off.size() <= 0xFFFE) {
         const auto t_claim = TClock::now();
-        k_claim_list<<<grid_for(ctx, ncand, 256), 256, 0, st>>>(cand, ncand, W, K, seed, block,
-                                                                recip, claim_list, d_norder, n,
-                                                                d_lover);
+        k_claim_list<<<blocks_for(ncand, 256 * kClaimPer), 256, 0, st>>>(
+            cand, ncand, W, K, seed, block, recip, claim_list, d_norder, n, d_lover);
         ctx->launches++;
         unsigned long long h_n[2] = {0, 0};
         u32 h_lover = 0;
@@ -929,10 +1165,8 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
         if (L == 0) break;
         S615_CU(cudaMemsetAsync(d_nnext, 0, 8, st));
         S615_CU(cudaMemsetAsync(d_lover, 0, 4, st));
-        k_apply_list<<<grid_for(ctx, (L + kApplyPer - 1) / kApplyPer, 256), 256, 0, st>>>(
-            claim_list.at(total), L, W, K, seed,
-                                                            block, recip,
-                                                            fr[cur ^ 1], d_nnext, fcap, d_lover);
+        k_apply_list<<<blocks_for(L, 256 * kApplyPer), 256, 0, st>>>(
+            claim_list.at(total), L, W, K, seed, block, recip, fr[cur ^ 1], d_nnext, fcap, d_lover);
         ctx->launches++;
         S615_CU(cudaGetLastError());
         S615_CU(cudaMemcpyAsync(&h_n[1], d_nnext, 8, cudaMemcpyDeviceToHost, st));
@@ -946,6 +1180,10 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
           cand = CellList{nullptr, nullptr};
           ncand = m;
           S615_CU(cudaMemsetAsync(d_lover, 0, 4, st));
+          if (claim_list.hash) {
+            k_zero_claimed<<<blocks_for(total, 256), 256, 0, st>>>(claim_list.cells, total, W, block);
+            ctx->launches++;
+          }
         } else {
           cand = fr[cur];
           ncand = h_n[1];
@@ -961,8 +1199,8 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
       trace.mark("peel");
       for (size_t q = off.size() - 1; q >= 1; --q) {
         const u64 L = off[q] - off[q - 1];
-        k_fill_list<<<grid_for(ctx, L, 256), 256, 0, st>>>(claim_list.at(off[q - 1]), L, W, K,
-                                                           seed, block, recip, mask);
+        k_fill_list<<<blocks_for(L, 256 * kFillPer), 256, 0, st>>>(claim_list.at(off[q - 1]), L, W, K,
+                                                                   seed, block, recip, mask);
         ctx->launches++;
       }
       trace_rounds = (int)off.size() - 1;
