@@ -773,8 +773,11 @@ struct Buf {
   void* p = nullptr;
   size_t n = 0;
   explicit Buf(s615_ctx* c) : ctx(c) {}
-  int alloc(size_t bytes) { n = bytes; return dev_alloc(ctx, &p, bytes); }
-  void release() { if (p) dev_free(ctx, p, n); p = nullptr; n = 0; }
+  bool own = true;
+  int alloc(size_t bytes) { n = bytes; own = true; return dev_alloc(ctx, &p, bytes); }
+  // n bytes of another buffer, which outlives this one
+  void view(void* at, size_t bytes) { release(); p = at; n = bytes; own = false; }
+  void release() { if (p && own) dev_free(ctx, p, n); p = nullptr; n = 0; }
   ~Buf() { release(); }
 };
 
@@ -865,8 +868,9 @@ int incidence_binned(s615_ctx* ctx, const u64* keys, u64 n, u64 seed, u64 m, u64
 // about 1.5 million keys, so that a slice's hash set (32 MB, and the next one's
 // being cleared) stays in L2; more and smaller ones when HBM is short, and
 // then as many passes over the source as the partition buffer needs.
-int unique_keys(s615_ctx* ctx, KeySource src, u64 n_raw, size_t avail, u64* out, u64 cap, u64* n,
-                cudaStream_t st) {
+// `given`, when it has room for every key, is used as the partition buffer.
+int unique_keys(s615_ctx* ctx, KeySource src, u64 n_raw, size_t avail, const Buf* given, u64* out,
+                u64 cap, u64* n, cudaStream_t st) {
   constexpr u64 kSliceKeys = 3ull << 19, kMost = 4096;
   u64 S = std::min<u64>(kMost, (n_raw + kSliceKeys - 1) / kSliceKeys);
   S = std::max<u64>(S, 1);
@@ -897,8 +901,9 @@ int unique_keys(s615_ctx* ctx, KeySource src, u64 n_raw, size_t avail, u64* out,
   // the partition buffer: every key when there is room, else what there is
   const size_t held = 2 * slots * 8 + PartScratch::bytes(G, S);
   const u64 room = avail > held ? (avail - held) / 8 : 0;
-  const u64 part_cap = std::max<u64>(std::min<u64>(all, room), std::max<u64>(most, 1));
-  if ((s = part.alloc(part_cap * 8))) return s;
+  u64 part_cap = std::max<u64>(std::min<u64>(all, room), std::max<u64>(most, 1));
+  if (given && given->n / 8 >= all) part.view(given->p, given->n), part_cap = given->n / 8;
+  else if ((s = part.alloc(part_cap * 8))) return s;
   auto* P = static_cast<unsigned long long*>(part.p);
   u32 flip = 0;
   for (u32 s0 = 0; s0 < S;) {
@@ -984,13 +989,39 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
   PhaseTrace trace(st);
   trace.mark("start");
   // ---- 1. unique keys ----
-  Buf keys(ctx);
+  // With room to spare, the scratch of the whole build is one allocation for
+  // at most n_raw keys: their array, the entry buffer (the partition's before
+  // the incidence, the claim list's after it), the candidate lists and the bin
+  // counts.  (Allocating and freeing 58 GB in five pieces for N = 48,000 took
+  // 50 to 150 ms of the build, with what had been freed just before.)
+  const size_t bin_bytes = PartScratch::bytes((size_t)ctx->num_sms * 2, kMaxSlices);
+  const u64 m_most = capacity_for(n_raw);
+  const auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  const size_t a_keys = up((n_raw + 1) * 8), a_ent = up(24 * (n_raw + 1)),
+               a_front = up(10 * std::max<u64>(4096, m_most / 8));
+  release_run_batch(ctx);   // a table needs the room more than s615_run's kept buffers
+  Buf arena(ctx), keys(ctx), ent(ctx), front(ctx), bins(ctx);
   u64 n = 0;
   {
+    size_t free_b = 0, total_b = 0;
+    S615_CU(cudaMemGetInfo(&free_b, &total_b));
+    const size_t all_bytes = a_keys + a_ent + a_front + up(bin_bytes);
+    if (n_raw < (1ull << 32) &&
+        std::min(free_b, budget_room(ctx)) > all_bytes + m_most * 8 + ((size_t)3 << 30) &&
+        !arena.alloc(all_bytes)) {
+      char* at = static_cast<char*>(arena.p);
+      keys.view(at, a_keys);
+      ent.view(at + a_keys, a_ent);
+      front.view(at + a_keys + a_ent, a_front);
+      bins.view(at + a_keys + a_ent + a_front, bin_bytes);
+    } else {
+      arena.p = nullptr;
+    }
+  }
+  {
     // +1: the all-ones key is kept out of the hash set and appended last
-    int s = keys.alloc((n_raw + 1) * sizeof(u64));
+    int s = arena.p ? 0 : keys.alloc((n_raw + 1) * sizeof(u64));
     if (s) return s;
-    release_run_batch(ctx);   // a table needs the room more than s615_run's kept buffers
     size_t free_b = 0, total_b = 0;
     S615_CU(cudaMemGetInfo(&free_b, &total_b));
     size_t avail = std::min(free_b, budget_room(ctx));
@@ -1004,7 +1035,9 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     src.shards = shards;
     src.shard = shard;
     src.srecip = mod_recip(shards);
-    if ((s = unique_keys(ctx, src, n_raw, avail, static_cast<u64*>(keys.p), n_raw, &n, st))) return s;
+    if ((s = unique_keys(ctx, src, n_raw, avail, arena.p ? &ent : nullptr, static_cast<u64*>(keys.p),
+                         n_raw, &n, st)))
+      return s;
   }
 
   std::memset(&out->hdr, 0, sizeof out->hdr);
@@ -1028,7 +1061,7 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
   S615_CU(cudaMemcpyToSymbolAsync(g_check_nkeys, &n, sizeof n, 0, cudaMemcpyHostToDevice, st));
   S615_CU(cudaMemcpyToSymbolAsync(g_check_ncells, &m, sizeof m, 0, cudaMemcpyHostToDevice, st));
 #endif
-  Buf cells(ctx), rounds(ctx), scratch(ctx), order(ctx), front(ctx);
+  Buf cells(ctx), rounds(ctx), scratch(ctx), order(ctx);
   int s = cells.alloc(m * sizeof(u64));
   if (s) return s;
   // Peel over lists (claimed cells in round order, two candidate lists of
@@ -1037,7 +1070,7 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
   // Candidate lists: two of m/8 entries (5 bytes each: offset + third).
   const u64 fcap = std::max<u64>(4096, m / 8);
   bool lists = block < (1ull << 32);
-  if (lists && front.alloc(2 * fcap * 5)) {
+  if (lists && !arena.p && front.alloc(2 * fcap * 5)) {
     front.release();
     lists = false;
   }
@@ -1062,19 +1095,19 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     const size_t margin = (size_t)2 << 30;
     return a > margin ? a - margin : 0;
   };
-  const size_t bin_bytes = PartScratch::bytes((size_t)ctx->num_sms * 2, kMaxSlices);
   // the recorded claim list needs 17 bytes per key in the entry buffers
   // (offset, third, u32 index, hash) and n < 2^32; otherwise the claimed
   // cells alone (5 bytes per key) are taken now, before the entry buffers
   const bool rich_possible = n < (1ull << 32);
-  if (lists && (!rich_possible || avail_now() < bin_bytes + 24 * n) && order.alloc(n * 5)) {
+  if (lists && !arena.p && (!rich_possible || avail_now() < bin_bytes + 24 * n) && order.alloc(n * 5)) {
     order.release(); front.release();
     lists = false;
   }
   if (!lists && (s = rounds.alloc(m * sizeof(u16)))) return s;
-  Buf ent(ctx), bins(ctx);   // ent: one 8-byte word per update (index << 32 | slice offset)
-  u64 ent_cap = 0;
-  {
+  u64 ent_cap = 0;   // of ent: one 8-byte word per update (index << 32 | slice offset)
+  if (arena.p) {
+    ent_cap = 3 * n;
+  } else {
     const size_t avail = avail_now();
     if (avail > bin_bytes) {
       ent_cap = std::min<u64>(3 * n, (avail - bin_bytes) / 8);
@@ -1240,9 +1273,9 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
   S615_CU(cudaStreamSynchronize(st));
   trace.mark("sync");
   keys.release(); rounds.release(); order.release(); front.release();
-  trace.mark("free_keys");
   ent.release(); bins.release();
-  trace.mark("free_bins");
+  arena.release();
+  trace.mark("free");
 
   out->hdr.n_keys = n;
   out->hdr.m_cells = m;
