@@ -16,6 +16,7 @@
 #include <cstring>
 #include <memory>
 #include <new>
+#include <numeric>
 #include <random>
 #include <thread>
 #include <vector>
@@ -31,30 +32,27 @@ int cuda_status(cudaError_t e) {
   return e == cudaSuccess ? S615_OK : S615_E_DEVICE;
 }
 
+int dev_alloc_once(s615_ctx* ctx, void** p, size_t bytes) {
+  *p = nullptr;
+  if (bytes == 0) bytes = 16;
+  // reserve the bytes against the budget first, so that threads allocating
+  // at once cannot overrun it together
+  size_t cur = ctx->used.load();
+  do {
+    if (ctx->budget && cur + bytes > ctx->budget) return S615_E_OOM;
+  } while (!ctx->used.compare_exchange_weak(cur, cur + bytes));
+  if (cudaMalloc(p, bytes) == cudaSuccess) return S615_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  ctx->used.fetch_sub(bytes);
+  return S615_E_OOM;
+}
+
 // A failed allocation gives back s615_run's kept batch, if it holds one that
 // no run is using, and tries once more.
 int dev_alloc(s615_ctx* ctx, void** p, size_t bytes) {
-  *p = nullptr;
-  if (bytes == 0) bytes = 16;
-  for (int attempt = 0;; ++attempt) {
-    // reserve the bytes against the budget first, so that threads allocating
-    // at once cannot overrun it together
-    bool reserved = false;
-    size_t cur = ctx->used.load();
-    while (!ctx->budget || cur + bytes <= ctx->budget) {
-      if (ctx->used.compare_exchange_weak(cur, cur + bytes)) {
-        reserved = true;
-        break;
-      }
-    }
-    if (reserved) {
-      if (cudaMalloc(p, bytes) == cudaSuccess) return S615_OK;
-      cudaGetLastError();
-      *p = nullptr;
-      ctx->used.fetch_sub(bytes);
-    }
-    if (attempt > 0 || !release_run_batch(ctx)) return S615_E_OOM;
-  }
+  if (dev_alloc_once(ctx, p, bytes) == S615_OK) return S615_OK;
+  return release_run_batch(ctx) ? dev_alloc_once(ctx, p, bytes) : S615_E_OOM;
 }
 
 void dev_free(s615_ctx* ctx, void* p, size_t bytes) {
@@ -79,6 +77,12 @@ bool release_run_batch(s615_ctx* ctx) {
     any = any || !ctx->pool.empty();
   }
   pool_release(ctx);
+  // the staged probe's space, unless another thread is launching with it
+  std::unique_lock<std::mutex> lock(ctx->stage.mu, std::try_to_lock);
+  if (lock.owns_lock() && ctx->stage.p) {
+    stage_release(ctx);
+    any = true;
+  }
   return any;
 }
 
@@ -881,6 +885,14 @@ static void run_threads(size_t nt, F&& work) {
   for (auto& x : th) x.join();
 }
 
+// About how many of a class 2-5 unit's points pass the gate (2.7% of the R > 0
+// points; a find3 row's window is about 0.15 lim long).
+static double est_keys(const DevUnit& d) {
+  if (d.cls == kClsJobRow) return d.w ? 0.03 : 0.004 * d.lim;
+  const double rows = (double)d.fmax1 / d.mod1 * d.nres1;
+  return rows * (d.cls == 5 ? 0.0243 * d.nres2 * d.fmax2 / 64 : 0.0043 * d.lim);
+}
+
 // make_dev_unit over every unit (on several host threads for large batches),
 // the kept records compacted in unit order.  Returns the error of the
 // lowest-index unit that has one, as a sequential pass would.
@@ -968,17 +980,21 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
     return d.cls == S615_CLS_617 || d.cls == 1 || d.cls == S615_CLS_617_FIND4;
   };
   std::vector<size_t> cnt_main(nt, 0), cnt_617(nt, 0);
+  std::vector<double> est(nt, 0.0);
   run_threads(nt, [&](size_t t) {
     ItemCount m, c;
+    double keys = 0;
     for (size_t k = cut[t]; k < cut[t + 1]; ++k) {
       const DevUnit& d = du[k];
       if (d.cls == 0) continue;   // dropped
       if (second(d)) unit_items(d, (u32)k, c, job_rows, unit_rows, b->parts3);
-      else unit_items(d, (u32)k, m, job_rows, unit_rows, b->parts3);
+      else unit_items(d, (u32)k, m, job_rows, unit_rows, b->parts3), keys += est_keys(d);
     }
     cnt_main[t] = m.n;
     cnt_617[t] = c.n;
+    est[t] = keys;
   });
+  b->est_keys = std::accumulate(est.begin(), est.end(), 0.0);
   std::vector<size_t> at(nt + 1, 0), at617(nt + 1, 0);
   for (size_t t = 0; t < nt; ++t) at[t + 1] = at[t] + cnt_main[t];
   at617[0] = at[nt];
@@ -1113,7 +1129,9 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
   };
   S615_CU(cudaMemsetAsync(b->d_ctr, 0, sizeof(Cls5Counters) + 64, st));
   if (!(flags & S615_F_PLAIN)) {
-    const int s = launch_peel(ctx, tv, b, flags, st, 0);
+    bool staged = false;
+    int s = launch_staged(ctx, tv, b, flags, st, &staged);
+    if (!s) s = launch_peel(ctx, tv, b, staged ? flags | kFlagNoMain : flags, st, 0);
     mark_done();
     return s;
   }

@@ -98,11 +98,18 @@ struct DevTable {
   void* d_views = nullptr;       // one TableView per shard of the set in HBM (owned ones set)
   u32 groups = 0;                // probe passes over a set (0: from its size)
   // The plane: the low 2^plane_lb bits of every cell, packed into 32-bit words
-  // (a single table whose plane fits L2 far better than its cells; table.cu).
+  // (a single table whose plane fits L2 far better than its cells, or, with
+  // plane_staged, one that the staged probe reads slice by slice; table.cu).
   void* d_plane = nullptr;
   size_t plane_bytes = 0;
   u32 plane_lb = 0;
+  bool plane_staged = false;
 };
+
+// The staged probe (staged.cu) reads a plane in slices; the largest may have
+// this many bytes and, with the pages that stream past, stay in L2 (scattered
+// reads keep their full rate up to a 64 MB footprint, 0.8 of it at 80 MB).
+constexpr u64 kStageSlice = 80ull << 20;
 
 // Random reads keep their rate over footprints up to 64 GiB and lose ~3x at
 // 110 GiB on a B200 (bin/randaccess_peak 2 8 29 64 110).  A shard set larger
@@ -112,6 +119,8 @@ constexpr u64 kProbeGroupBytes = 56ull << 30;
 // Internal launch flag: a pass after the first adds no counters (it repeats
 // the first pass's points; only its probes differ).
 constexpr unsigned kFlagNoCount = 1u << 30;
+// Internal launch flag: the classes 2-5 items have been run already.
+constexpr unsigned kFlagNoMain = 1u << 29;
 
 // Kernel-facing view of a table (or of a shard set: shards > 1, parts).
 struct TableView {
@@ -124,6 +133,7 @@ struct TableView {
   u32 groups, pad;      // passes over the set
   u64 bytes;            // bytes of cells (a single table; 0 for a set)
   const u32* plane;     // low 2^plane_lb bits of each cell (null: none)
+  const u32* splane;    // the same, for the staged probe only
   u64 plane_bytes;
   u32 plane_lb, plane_mask;   // plane_mask = 2^(2^plane_lb) - 1
 };
@@ -186,6 +196,7 @@ struct s615_batch {
   // part): part p sieves every parts3-th 1024-column tile of the rows' c3 windows
   s615::u32 parts3 = 1;
   s615::u32 blocks_per_sm = 0;              // k_peel blocks per SM (0: the occupancy limit)
+  double est_keys = 0;          // about how many keys of classes 2-5 pass the gate
   cudaEvent_t done = nullptr;   // recorded after the last s615_run_batch's launches
   // host copy of the work items: grow-only and uninitialised, written in
   // place by the fill's threads
@@ -194,6 +205,16 @@ struct s615_batch {
 };
 
 namespace s615 {
+// The staged probe's pages and chunk counters: one space per context, handed
+// from run to run (on any stream) through the event; given back with
+// s615_run's kept batch.
+struct StageSpace {
+  std::mutex mu;
+  void* p = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t last = nullptr;   // recorded after the last run that used it
+};
+
 // A grow-only host buffer: pinned when the driver grants it, pageable if not.
 struct HostStage {
   void* p = nullptr;
@@ -240,6 +261,7 @@ struct s615_ctx {
   size_t pool_bytes = 0;
   std::mutex pool_mu;
   bool run_busy = false;
+  s615::StageSpace stage;
   // L2-persisting access windows (cudaDevAttrMaxPersistingL2CacheSize,
   // cudaDevAttrMaxAccessPolicyWindowSize) and the set-aside this context
   // has asked for (cudaLimitPersistingL2CacheSize, per process).
@@ -268,7 +290,9 @@ void stage_free(HostStage& s);
 // freed batch buffers; true if either held anything.
 bool release_run_batch(s615_ctx* ctx);
 
-// Budgeted device allocation.
+// Budgeted device allocation.  dev_alloc_once neither gives anything back nor
+// tries again when there is no room.
+int dev_alloc_once(s615_ctx* ctx, void** p, size_t bytes);
 int dev_alloc(s615_ctx* ctx, void** p, size_t bytes);
 void dev_free(s615_ctx* ctx, void* p, size_t bytes);
 // Batch buffers through the context's pool: pool_get hands out a pooled
@@ -305,6 +329,11 @@ int l2_window(s615_ctx* ctx, const TableView& tv, unsigned flags, cudaLaunchAttr
 // kernel over [n_main, n_items), in that order on st.
 int launch_peel(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                 cudaStream_t st, int grid_blocks);
+// Probes the batch's classes 2-5 items in stages when that is the faster way
+// (*done = true: launch_peel then gets kFlagNoMain).  The caller holds nothing.
+int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
+                  cudaStream_t st, bool* done);
+void stage_release(s615_ctx* ctx);   // the caller holds ctx->stage.mu
 int launch_peel617(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                    cudaStream_t st, int grid_blocks);
 // Builds t's plane when it would make the probe cheaper (and the HBM budget

@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "peel_common.cuh"
+#include "staged.cuh"
 
 namespace s615 {
 
@@ -80,6 +81,18 @@ struct PeelParams {
   u32 count;               // add this launch's counters (0 for a repeat pass over a set)
   u32 item_rows;           // rows per item of the batch (<= kRows)
   u32 parts3_log2;         // log2 of the items per class 2-4 row chunk (1 or 4 items)
+  u32 item_lo;             // first item of this launch (its items: [item_lo, n_items))
+  u32 sub_log2;            // each item goes out as 2^sub_log2 parts of its rows
+  u32 sb;                  // kEmit: a bucket is 2^sb cells
+  StagePages pages;        // kEmit: where keys go
+  StageChunk* chunk;       // kEmit, kResolve
+};
+
+// What a full batch of gate survivors meets.
+enum : int {
+  kProbe = 0,     // the xor probe, hits recorded
+  kEmit = 1,      // the staged probe's first step: keys to pages by first cell
+  kResolve = 2,   // its last: the probe again, for the keys in the chunk's Bloom filter
 };
 
 // cls5 pattern words (sharp or not) then the find3 ones, then the warp slices
@@ -88,8 +101,11 @@ template <bool kSharp>
 constexpr size_t smem_pat() {
   return ((size_t)((kSharp ? kSharpWords : kPatWords) + kPatWords) * sizeof(u32) + 15) / 16 * 16;
 }
-template <bool kSharp>
-constexpr size_t smem_total() { return smem_pat<kSharp>() + kWarps * sizeof(WarpT<kSharp>); }
+template <bool kSharp, int kMode>
+constexpr size_t smem_total() {
+  return smem_pat<kSharp>() + kWarps * (sizeof(WarpT<kSharp>) + (kMode == kEmit ? sizeof(WarpHold) : 0));
+}
+static_assert(sizeof(WarpSmem) % 8 == 0, "the held keys follow the warp slices");
 
 // x^6 mod 512 for small x.
 __device__ __forceinline__ u32 pow6_mod512(u32 x) {
@@ -106,10 +122,37 @@ struct ItemCtx {
   u32 cls, unit_id, r0, mod, j0, f;   // job items: unit_id = index of the first unit
 };
 
+// kEmit: a key whose bucket has no page left is probed where it is.
+struct DirectProbe {
+  const TableView& tv;
+  StageChunk* chunk;
+  __device__ __forceinline__ void operator()(u32, u64 h) const {
+    if (contains_hash<false>(tv, h)) stage_positive(chunk, h);
+  }
+};
+
 // Probe the ring entries [head, head+cnt) (one per lane).
-template <bool kSet>
+template <bool kSet, int kMode>
 __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem& W, u32 head,
-                                            u32 cnt, const ItemCtx& I, u32 lane) {
+                                            u32 cnt, const ItemCtx& I, u32 lane, StageOpen& S,
+                                            WarpHold* H) {
+  if constexpr (kMode == kEmit) {
+    const bool act = lane < cnt;
+    u64 h = 0;
+    u32 b = 0;
+    if (act) {
+      const u32 ent = W.ring[(head + lane) & (kQ - 1)];
+      const u32 k = ent & 0x3FFFFu, r = (ent >> 18) & 63u, di = ent >> 24;
+      const RowRec& R = W.rows[r];
+      u64 key;
+      if (I.cls == 5) key = (u64)(((((u128)R.whi << 64) | R.wlo) - pow6_small((u64)W.d0s[di] + 64ull * k)) >> 6);
+      else key = R.wlo - (u64)pow6_small((u64)R.a + k);
+      h = mix64(key + P.tv.seed);
+      b = (u32)(fast_mod(h, P.tv.block, P.tv.recip) >> P.sb);
+    }
+    stage_push(P.pages, *H, S, act, b, h, lane, DirectProbe{P.tv, P.chunk});
+    return;
+  }
   if (lane >= cnt) return;
   const u32 ent = W.ring[(head + lane) & (kQ - 1)];
   const u32 k = ent & 0x3FFFFu, r = (ent >> 18) & 63u, di = ent >> 24;
@@ -125,6 +168,10 @@ __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem&
     x = (u64)R.a + k;                               // c3
     key = R.wlo - (u64)pow6_small(x);               // T - c3^6 mod 2^64
     rowval = I.r0 + I.mod * (I.j0 + r);             // d
+  }
+  if constexpr (kMode == kResolve) {
+    const u32 bit = (u32)(mix64(key + P.tv.seed) >> (64 - kBloomBits));
+    if (!((__ldcg(&P.chunk->bloom[bit >> 5]) >> (bit & 31u)) & 1u)) return;
   }
   if (probe_table<kSet>(P.tv, key)) {
     const unsigned long long idx = atomicAdd(&P.ctr->hits, 1ull);
@@ -145,10 +192,10 @@ __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem&
 }
 
 // Push the set bits of m into the ring; probe every full batch of 32.
-template <bool kSet>
+template <bool kSet, int kMode>
 __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 m, u32 di, u32 r,
                                           u32 kbase, u32& head, u32& qlen, const ItemCtx& I,
-                                          u32 lane) {
+                                          u32 lane, StageOpen& S, WarpHold* H) {
   while (__any_sync(0xFFFFFFFFu, m != 0)) {
     const bool has = m != 0;
     const u32 bit = has ? (u32)(__ffs(m) - 1) : 0u;
@@ -158,7 +205,7 @@ __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 
     qlen += __popc(ballot);
     if (qlen >= 32u) {
       __syncwarp();
-      probe_batch<kSet>(P, W, head, 32u, I, lane);
+      probe_batch<kSet, kMode>(P, W, head, 32u, I, lane, S, H);
       __syncwarp();
       head = (head + 32u) & (kQ - 1);
       qlen -= 32u;
@@ -166,9 +213,12 @@ __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 
   }
 }
 
-template <bool kSharp, bool kSet>
-__global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P) {
+template <bool kSharp, bool kSet, int kMode = kProbe>
+__global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5) k_peel(PeelParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
+  if constexpr (kMode == kResolve) {
+    if (P.chunk->positives == 0) return;   // nothing in this chunk: the usual case
+  }
   constexpr u32 kP5 = kSharp ? (u32)kSharpWords : (u32)kPatWords;
   u32* s_pat5 = reinterpret_cast<u32*>(smem);
   u32* s_pat3 = s_pat5 + kP5;
@@ -180,11 +230,17 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
 
   const u128 inv21 = ((u128)P.inv21_hi << 64) | P.inv21_lo;
   u64 my_calls = 0, my_pos = 0, my_probes = 0;
+  StageOpen S;
+  WarpHold* H = nullptr;
+  if constexpr (kMode == kEmit)
+    H = reinterpret_cast<WarpHold*>(smem + smem_pat<kSharp>() + kWarps * sizeof(WarpT<kSharp>)) + warp;
 
   for (;;) {
     u32 it = 0;
     if (lane == 0) it = atomicAdd(P.work, 1u);
     it = __shfl_sync(0xFFFFFFFFu, it, 0);
+    const u32 part = it & ((1u << P.sub_log2) - 1u);   // this part of the item's rows
+    it = (it >> P.sub_log2) + P.item_lo;
     if (it >= P.n_items) break;
     const u64 packed = P.items[it];
     if (!S615_CHECK(item_unit(packed) < P.n_units, kChkItem)) continue;   // warp-uniform
@@ -200,6 +256,11 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
       I.j0 = 0;
       nrows = job_count(packed);
       if (!S615_CHECK(item_unit(packed) + nrows <= P.n_units, kChkItem)) continue;
+      const u32 each = (nrows + (1u << P.sub_log2) - 1u) >> P.sub_log2, row0 = part * each;
+      if (row0 >= nrows) continue;
+      nrows = min(each, nrows - row0);
+      U += row0;
+      I.unit_id += row0;
     } else {
       if (!S615_CHECK(item_res(packed) < U->nres1 && U->nres1 <= 24, kChkItem)) continue;
       I.r0 = U->res1[item_res(packed)];
@@ -211,8 +272,10 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
         if (lane == 0) { W.part = ch & ((1u << P.parts3_log2) - 1u); W.nparts = 1u << P.parts3_log2; }
         ch >>= P.parts3_log2;
       }
-      I.j0 = jmin + ch * P.item_rows;
-      nrows = min(P.item_rows, jend - I.j0);
+      const u32 each = (P.item_rows + (1u << P.sub_log2) - 1u) >> P.sub_log2, row0 = part * each;
+      I.j0 = jmin + ch * P.item_rows + row0;
+      if (row0 >= P.item_rows || I.j0 >= jend) continue;
+      nrows = min(min(each, P.item_rows - row0), jend - I.j0);
     }
     if (I.cls == kClsJobRow && lane == 0) { W.part = 0; W.nparts = 1; }
     u32 head = 0, qlen = 0;
@@ -313,12 +376,12 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
                 m &= lowmask;
               }
               my_probes += __popc(m);
-              push_bits<kSet>(P, W, m, di, r, kbase, head, qlen, I, lane);
+              push_bits<kSet, kMode>(P, W, m, di, r, kbase, head, qlen, I, lane, S, H);
             }
           }
         }
         __syncwarp();
-        probe_batch<kSet>(P, W, head, qlen, I, lane);   // drain before d0s change
+        probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, S, H);   // drain before d0s change
         head = 0;
         qlen = 0;
         __syncwarp();
@@ -395,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
           }
         }
         my_probes += __popc(m);
-        push_bits<kSet>(P, W, m, 0, rr & 63u, kbase, head, qlen, I, lane);
+        push_bits<kSet, kMode>(P, W, m, 0, rr & 63u, kbase, head, qlen, I, lane, S, H);
         if (find2) {
           r += 32;
         } else if ((wt += W.nparts) >= (len + 1023u) / 1024u) {   // len: the same in every lane
@@ -404,10 +467,12 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
         }
       }
       __syncwarp();
-      probe_batch<kSet>(P, W, head, qlen, I, lane);
+      probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, S, H);
       __syncwarp();
     }
   }
+
+  if constexpr (kMode == kEmit) stage_close(P.pages, *H, S, lane, DirectProbe{P.tv, P.chunk});
 
   // ---- counters: warp reduce, one atomic per warp ----
 #pragma unroll
@@ -423,16 +488,21 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : 5) k_peel(PeelParams P)
   }
 }
 
-// k_peel over items [0, n) of the batch.
-template <bool kSharp, bool kSet>
+// k_peel over items [0, n) of the batch, or for the staged probe over [sl->lo, n).
+struct StageLaunch {
+  u32 lo, sb;
+  StagePages pages;
+  StageChunk* chunk;
+};
+template <bool kSharp, bool kSet, int kMode = kProbe>
 int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t n,
-                unsigned flags, cudaStream_t st, int grid_blocks) {
+                unsigned flags, cudaStream_t st, int grid_blocks, const StageLaunch* sl = nullptr) {
   // the shared-memory attribute belongs to each device's context: one bit per device
   static std::atomic<unsigned long long> attr_set{0};
-  constexpr size_t kSmemTotal = smem_total<kSharp>();
+  constexpr size_t kSmemTotal = smem_total<kSharp, kMode>();
   const unsigned long long dev_bit = 1ull << (ctx->device & 63);
   if (!(attr_set.load() & dev_bit)) {
-    S615_CU(cudaFuncSetAttribute(k_peel<kSharp, kSet>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    S615_CU(cudaFuncSetAttribute(k_peel<kSharp, kSet, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kSmemTotal));
     attr_set.fetch_or(dev_bit);
   }
@@ -459,15 +529,29 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
   P.inv21_lo = (u64)inv;
   P.inv21_hi = (u64)(inv >> 64);
   P.s8 = gated ? 0x7u : 0xFFu;
+  if (kMode != kProbe) {
+    P.item_lo = sl->lo;
+    P.sb = sl->sb;
+    P.pages = sl->pages;
+    P.chunk = sl->chunk;
+    P.work = sl->chunk->work[kMode == kEmit ? 0 : 4];
+  }
   if (n == 0) return S615_OK;
   int grid = grid_blocks;
   if (grid <= 0) {
     int per_sm = 0;
-    S615_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel<kSharp, kSet>, kThreads, kSmemTotal));
+    S615_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel<kSharp, kSet, kMode>, kThreads, kSmemTotal));
     if (b->blocks_per_sm && (int)b->blocks_per_sm < per_sm) per_sm = (int)b->blocks_per_sm;
     grid = ctx->num_sms * (per_sm > 0 ? per_sm : 1);
   }
-  const size_t need = (n + kWarps - 1) / kWarps;
+  // The staged probe's passes deal items out in parts, until each warp has 16 of
+  // them to take or a part is down to 256 keys (its row set-up then shows).
+  const u64 n_here = n - P.item_lo, warps = (u64)grid * kWarps;
+  const double per_item = b->est_keys / (double)std::max<size_t>(b->n_main, 1);
+  while (kMode != kProbe && P.sub_log2 < 4 && (n_here << P.sub_log2) < warps * 16 &&
+         per_item >= (double)(512u << P.sub_log2))
+    ++P.sub_log2;
+  const size_t need = ((n_here << P.sub_log2) + kWarps - 1) / kWarps;
   if ((size_t)grid > need) grid = (int)need;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
@@ -477,7 +561,7 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
   cudaLaunchAttribute attr[1];
   cfg.attrs = attr;
   cfg.numAttrs = (unsigned)l2_window(ctx, tv, flags, attr);
-  S615_CU(cudaLaunchKernelEx(&cfg, k_peel<kSharp, kSet>, P));
+  S615_CU(cudaLaunchKernelEx(&cfg, k_peel<kSharp, kSet, kMode>, P));
   ctx->launches++;
   S615_CU(cudaGetLastError());
   return S615_OK;
@@ -487,7 +571,7 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
 
 static int launch_pass(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                        cudaStream_t st, int grid_blocks) {
-  if (b->n_main) {
+  if (b->n_main && !(flags & kFlagNoMain)) {
     const bool sharp = (flags & S615_F_SHARP) && !(flags & S615_F_NO_GATE);
     const bool set = tv.shards > 1;
     const int s =
@@ -519,6 +603,14 @@ int launch_peel(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flag
     if (s) return s;
   }
   return S615_OK;
+}
+
+int launch_stage_peel(s615_ctx* ctx, const TableView& tv, const s615_batch* b, unsigned flags,
+                      cudaStream_t st, bool resolve, u32 lo, u32 hi, u32 sb, const StagePages& pages,
+                      StageChunk* chunk) {
+  const StageLaunch sl{lo, sb, pages, chunk};
+  return resolve ? launch_main<false, false, kResolve>(ctx, tv, b, hi, flags | kFlagNoCount, st, 0, &sl)
+                 : launch_main<false, false, kEmit>(ctx, tv, b, hi, flags, st, 0, &sl);
 }
 
 S615_CHECK_TAKE_DEFINE(check_take_peel)

@@ -115,9 +115,7 @@ __device__ __forceinline__ u32 load_plane(const TableView& t, u64 i) {
 // the shards of a set, which have none; the check costs k_peel's set instance
 // spills.)
 template <bool kPlane>
-__device__ __forceinline__ bool might_contain_one(const TableView& t, u64 key) {
-  if (t.block == 0) return false;
-  const u64 h = mix64(key + t.seed);
+__device__ __forceinline__ bool contains_hash(const TableView& t, u64 h) {
   u64 c[3];
   cell_indices(h, t.block, t.recip, c);
   if (!S615_CHECK(c[0] < 3 * t.block && c[1] < 3 * t.block && c[2] < 3 * t.block, kChkCell))
@@ -133,6 +131,11 @@ __device__ __forceinline__ bool might_contain_one(const TableView& t, u64 key) {
   const u64 b = load_cell(t, c[1]);
   const u64 d = load_cell(t, c[2]);
   return (a ^ b ^ d) == (h & t.fpmask);
+}
+
+template <bool kPlane>
+__device__ __forceinline__ bool might_contain_one(const TableView& t, u64 key) {
+  return t.block != 0 && contains_hash<kPlane>(t, mix64(key + t.seed));
 }
 
 // A shard set sends the probe to the key's own shard, mix64(key + seed) % S

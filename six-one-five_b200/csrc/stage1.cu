@@ -191,6 +191,10 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
   u64 n_units = 0;
   for (u32 i = 0; i < nB; ++i) { off[i] = (u32)n_units; n_units += counts[i]; }
   if (n_units > kMaxBatchUnits) return S615_E_ARG;
+  for (u32 i = 0; i < nB; ++i) {   // keys past the gate: 24 residue pairs of (B/14) x (B/21), 2.43%
+    const double B = (double)(B_lo + i);
+    b->est_keys += counts[i] * B * B * (24.0 / 46656 / 294 * 0.0243);
+  }
   S615_CU(cudaMemcpyAsync(d_off, off.data(), nB * 4, cudaMemcpyHostToDevice, st));
   // 2. the batch's unit records and item counts
   const size_t nu = std::max<size_t>(n_units, 1);

@@ -1,0 +1,388 @@
+// staged.cu -- the staged probe: large batches against tables past L2.
+//
+// A probe reads three scattered cells, and a B200 fills at most 4.7e10 of
+// them a second from DRAM (21 ps each, 64 of the 64 ps a class-5 probe of the
+// 3.2M band takes; the sieve itself is 7 ps).  From L2 the same reads take 3.5
+// ps.  So a large batch is probed in chunks, in steps that each read a part
+// of the table that stays in L2:
+//
+//   emit     the peel and the gate (k_peel) write each surviving key's hash to
+//            a page of its bucket: the slice of the first third its cell lies in;
+//   stage 1  page by page in bucket order, the low four bits of the first cell
+//            are read from the table's plane (a 17th to a 32nd of a third: 38 MB
+//            at most for N = 76,667) and the key goes on, with them, to a page
+//            by the slice of its second cell;
+//   stage 2  the same with the second and third cells;
+//   stage 3  the third cell's low bits complete the comparison of the low bits;
+//            one key in 16 passes and its cells are read in full.  A key that
+//            the table holds sets its bit in the chunk's Bloom filter;
+//   resolve  only if the chunk has such a key (a false positive of the filter
+//            included): the peel runs over the chunk once more and probes the
+//            keys whose bit is set, recording hits as ever.
+//
+// The comparison is the probe's own, cut in parts, so hits and counters are the
+// direct probe's.  A key whose bucket has no page left is probed where it is.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "staged.cuh"
+
+namespace s615 {
+
+int launch_stage_peel(s615_ctx* ctx, const TableView& tv, const s615_batch* b, unsigned flags,
+                      cudaStream_t st, bool resolve, u32 lo, u32 hi, u32 sb, const StagePages& pages,
+                      StageChunk* chunk);
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kPer = 4;        // keys per thread and pass
+
+struct StageParams {
+  TableView tv;
+  const u32* plane;
+  u32 sb;
+  StagePages first;   // step 1's input
+  StageRuns in, out;  // the others'
+  StageChunk* chunk;
+};
+
+constexpr u32 kPlaneLb = 2;    // 4 bits of each cell, eight cells to a word
+
+// A step's input as units of kUnit entries of one bucket (pages follow one
+// another in a bucket, and a piece is a multiple of a unit): warp-wide state.
+template <int kStep, u32 kUnit>
+struct UnitOrder {
+  u32 incl, n, total;
+  __device__ __forceinline__ UnitOrder(const StageParams& P, u32 lane) {
+    n = 0;
+    if (kStep == 1 ? lane < P.first.nb : lane < P.in.nb)
+      n = kStep == 1 ? (min(P.first.npages[lane * kStageStride], P.first.cap) + kUnit / kStagePage - 1) /
+                           (kUnit / kStagePage)
+                     : (min(P.in.count[lane * kStageStride], P.in.cap) + kUnit - 1) / kUnit;
+    incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= (u32)o) incl += y;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+  }
+  // Unit g < total: its bucket, first entry and length (step 1: its pages'
+  // entries, whatever their fills).
+  __device__ __forceinline__ void at(const StageParams& P, u32 g, u32& b, u64& e, u32& len) const {
+    b = __popc(__ballot_sync(0xFFFFFFFFu, incl <= g));   // buckets wholly before unit g
+    const u32 i = (g - __shfl_sync(0xFFFFFFFFu, incl - n, b)) * kUnit;
+    if constexpr (kStep == 1) {
+      e = (u64)b * P.first.cap * kStagePage + i;
+      len = min(min(P.first.npages[b * kStageStride], P.first.cap) * kStagePage - i, kUnit);
+    } else {
+      e = P.in.at(b, i);
+      len = min(min(P.in.count[b * kStageStride], P.in.cap) - i, kUnit);
+    }
+  }
+};
+
+// Cell kStep - 1 of an entry of bucket b: its index in the table, and its word g.
+template <int kStep>
+__device__ __forceinline__ u64 stage_open(const StageParams& P, u64 e, u32 b, u64& g) {
+  const u32 block = (u32)P.tv.block;
+  if constexpr (kStep == 1) {   // entries are the hashes
+    g = e;
+    u64 q;
+    u32 off;
+    split_word(e, block, P.tv.recip, q, off);
+    return off;
+  } else {
+    g = entry_word(e, b, P.sb, block);
+    return (u64)(kStep - 1) * block + ((b << P.sb) | ((u32)(e >> 4) & ((1u << P.sb) - 1u)));
+  }
+}
+__device__ __forceinline__ u32 plane_bits(u32 w, u64 c) { return w >> (((u32)c & 7u) << kPlaneLb); }
+
+// Steps 1 and 2: look cell kStep - 1 up and send the key on by cell kStep.  The
+// block orders 1,024 keys by bucket in shared memory and appends each bucket's
+// run (some 30 to 60 keys) to the bucket.
+//
+// Scattered accesses run at full rate only while they stay within some 16
+// regions of 16 MB, the reach of the first-level TLB (8 MB of lines in L2 read
+// at 2.8e11/s within 128 MB, at 4.5e10/s spread over 1 GB), so input, output and
+// plane slice are laid out to lie within that (StageRuns).  With a page per
+// warp and bucket, each bucket in a region of its own, a step took 23 ps a key.
+//
+// A block always knows its next unit: the queue's answer and the buckets' new
+// ends come back while it works.
+template <int kStep>
+__global__ void __launch_bounds__(kThreads, 5) k_stage(StageParams P) {
+  constexpr u32 kNone = 0xFFFFFFFFu, kUnit = kThreads * kPer;
+  __shared__ unsigned long long s_e[kUnit];
+  __shared__ u8 s_b[kUnit];
+  __shared__ u32 s_cnt[kStageBuckets], s_off[kStageBuckets], s_dst[kStageBuckets];
+  __shared__ u32 s_fill[kPer];
+  __shared__ u64 s_at;
+  __shared__ u32 s_in, s_len, s_total;
+  const u32 tid = threadIdx.x, lane = tid & 31;
+  const unsigned long long* in = kStep == 1 ? P.first.e : P.in.e;
+  const u32 block = (u32)P.tv.block, sb = P.sb;
+  const u64 recip = P.tv.recip;
+  const UnitOrder<kStep, kUnit> O(P, lane);
+  // warp 0: unit g's place to shared memory (s_len = 0: no more units)
+  auto place = [&](u32 g) {
+    u32 b = 0, len = 0;
+    u64 e = 0;
+    if (g < O.total) O.at(P, g, b, e, len);
+    if (kStep == 1 && lane < (u32)kPer) {
+      const u64 page = e / kStagePage + lane;
+      s_fill[lane] = lane * kStagePage < len ? min(P.first.fill[page], kStagePage) : 0u;
+    }
+    if (lane == 0) { s_at = e; s_in = b; s_len = len; }
+  };
+  u32 next = 0;
+  if (tid < 32) {
+    if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+    place(__shfl_sync(0xFFFFFFFFu, next, 0));
+    if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+    s_cnt[lane] = 0;
+  }
+  for (;;) {
+    __syncthreads();
+    const u32 len = s_len, ib = s_in;
+    if (len == 0) break;
+    const unsigned long long* src = in + s_at;
+    u64 g[kPer];
+    u32 w[kPer], x[kPer], at[kPer], act = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const u32 i = (u32)k * kThreads + tid;
+      const bool on = kStep == 1 ? tid < s_fill[k] : i < len;
+      g[k] = on ? (u64)__ldcs(src + i) : 0;
+      act |= (u32)on << k;
+    }
+    // the plane's answers come back while the next words are worked out
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const u32 e = (u32)g[k];
+      const u64 c = stage_open<kStep>(P, g[k], ib, g[k]);
+      x[k] = (e & 15u) | ((u32)c & 7u) << 6;   // low bits so far | 4 * (cell % 8)
+      w[k] = (act >> k) & 1u ? __ldcg(P.plane + (c >> (5 - kPlaneLb))) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      u64 q;
+      u32 off;
+      split_word(cell_word<kStep>(hash_of_word<kStep - 1>(g[k])), block, recip, q, off);
+      g[k] = pack_entry(q, off, sb, 0);
+      const u32 b = off >> sb;
+      at[k] = ((act >> k) & 1u) ? b | (atomicAdd(&s_cnt[b], 1u) << 5) : kNone;
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) g[k] |= (x[k] ^ (w[k] >> (x[k] >> 4))) & 15u;
+    __syncthreads();
+    u32 base = 0, off0 = 0;
+    if (tid < 32) {   // the runs' places: lane b for bucket b
+      const u32 r = s_cnt[lane];
+      if (r) base = atomicAdd(P.out.count + lane * kStageStride, r);
+      s_cnt[lane] = 0;
+      u32 incl = r;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (u32)o) incl += y;
+      }
+      off0 = incl - r;
+      s_off[lane] = off0;
+      if (lane == 31) s_total = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (at[k] != kNone) {
+        const u32 b = at[k] & 31u, pos = s_off[b] + (at[k] >> 5);
+        s_e[pos] = g[k];
+        s_b[pos] = (u8)b;
+      }
+    if (tid < 32) {
+      place(__shfl_sync(0xFFFFFFFFu, next, 0));
+      if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+      s_dst[lane] = base - off0;   // entry i of the tile goes to place s_dst + i
+    }
+    __syncthreads();
+    const u32 total = s_total;
+    for (u32 pos = tid; pos < total; pos += kThreads) {
+      const u32 b = s_b[pos], i = s_dst[b] + pos;
+      const u64 e = s_e[pos];
+      if (i < P.out.cap) {
+        P.out.e[P.out.at(b, i)] = e;
+      } else {   // no room left in the bucket: probed here
+        const u64 h = hash_of_word<kStep>(entry_word(e, b, sb, block));
+        if (contains_hash<false>(P.tv, h)) stage_positive(P.chunk, h);
+      }
+    }
+  }
+}
+
+// Step 3: the last cell's low bits; one key in 16 agrees and is probed in full.
+// Warps take units of 1,024 keys, eight keys a lane in flight.
+constexpr u32 kTake = 1024;
+__global__ void __launch_bounds__(kThreads) k_stage_last(StageParams P) {
+  const u32 lane = threadIdx.x & 31;
+  const UnitOrder<3, kTake> O(P, lane);
+  u32 next = 0;
+  if (lane == 0) next = atomicAdd(P.chunk->work[3], 1u);
+  for (;;) {
+    const u32 unit = __shfl_sync(0xFFFFFFFFu, next, 0);
+    if (unit >= O.total) break;
+    if (lane == 0) next = atomicAdd(P.chunk->work[3], 1u);
+    u32 b, len;
+    u64 at;
+    O.at(P, unit, b, at, len);
+    for (u32 i0 = 0; i0 < len; i0 += 256u) {
+      u64 e[8];
+      u32 x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const u32 i = i0 + 32u * k + lane;
+        e[k] = i < len ? (u64)__ldcs(P.in.e + at + i) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const u64 c = 2 * P.tv.block + ((u64)b << P.sb) + ((e[k] >> 4) & ((1ull << P.sb) - 1));
+        const bool on = i0 + 32u * k + lane < len;
+        x[k] = on ? (u32)e[k] ^ plane_bits(__ldcg(P.plane + (c >> (5 - kPlaneLb))), c) : 1u;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (!(x[k] & 15u)) {
+          const u64 h = hash_of_word<2>(entry_word(e[k], b, P.sb, (u32)P.tv.block));
+          if (contains_hash<false>(P.tv, h)) stage_positive(P.chunk, h);
+        }
+    }
+  }
+}
+
+template <class K>
+int launch_stage(s615_ctx* ctx, K kernel, const StageParams& P, cudaStream_t st) {
+  int per_sm = 0;
+  S615_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+  kernel<<<ctx->num_sms * std::max(per_sm, 1), kThreads, 0, st>>>(P);
+  ctx->launches++;
+  S615_CU(cudaGetLastError());
+  return S615_OK;
+}
+
+// Most warps of any of the kernels that write pages (each may leave a page
+// part-filled in every bucket).
+u64 stage_warps(const s615_ctx* ctx) { return (u64)ctx->num_sms * 64; }
+
+// Keys per chunk: enough that reading the plane once per chunk and the ends of
+// six launches are small beside it, few enough that most chunks of a search hold
+// no key of the table (about one in 1e9) and skip the resolve pass.
+constexpr u64 kMaxChunkKeys = 1ull << 28, kMinChunkKeys = 1ull << 26;
+constexpr double kMinKeys = 1e8;
+
+// Two spaces in turn: the emitted pages, stage 1's runs, stage 2's in the
+// pages' place.
+struct Layout {
+  u32 nb = 0, pages = 0, entries = 0;   // per bucket: pages emitted, entries of a run
+  size_t first = 0, second = 0, bytes = 0;
+};
+Layout layout_for(const s615_ctx* ctx, u64 keys, u32 nb) {
+  Layout L;
+  L.nb = nb;
+  const u64 each = (keys + keys / 8) / nb;
+  L.pages = (u32)(each / kStagePage + stage_warps(ctx));
+  L.entries = (u32)((each >> kStagePieceLog2) + 1) << kStagePieceLog2;
+  L.second = (size_t)nb * L.entries * 8;
+  L.first = std::max(L.second, (size_t)nb * L.pages * (kStagePage * 8 + 4));
+  L.first = (L.first + 255) / 256 * 256;
+  L.bytes = (sizeof(StageChunk) + 255) / 256 * 256 + L.first + L.second;
+  return L;
+}
+
+}  // namespace
+
+void stage_release(s615_ctx* ctx) {
+  StageSpace& w = ctx->stage;
+  if (w.last) {
+    cudaEventSynchronize(w.last);
+    cudaEventDestroy(w.last);
+    w.last = nullptr;
+  }
+  dev_free(ctx, w.p, w.bytes);
+  w.p = nullptr;
+  w.bytes = 0;
+}
+
+// *done = true when the classes 2-5 items of b were probed in stages.
+int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags, cudaStream_t st,
+                  bool* done) {
+  *done = false;
+  double est = b->est_keys;
+  if (flags & S615_F_NO_GATE) est *= 37;   // 2.7% of the points pass the gate
+  if (!tv.splane || tv.shards > 1 || (flags & S615_F_SHARP) || est < kMinKeys || !b->n_main)
+    return S615_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return S615_OK;
+  }
+  std::lock_guard<std::mutex> lock(ctx->stage.mu);
+  StageSpace& w = ctx->stage;
+  // chunks of at most kMaxChunkKeys keys, smaller when HBM is short
+  u64 keys = (u64)std::min<double>(est * 1.05, (double)kMaxChunkKeys);
+  const u32 sb = stage_shift(tv.block);
+  const u32 nb = (u32)((tv.block + (1ull << sb) - 1) >> sb);
+  Layout L = layout_for(ctx, keys, nb);
+  if (L.bytes > w.bytes) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
+    const size_t used = ctx->used.load();
+    const size_t room = w.bytes + std::min(free_b, ctx->budget > used ? ctx->budget - used : 0) / 4;
+    while (L.bytes > room && keys > kMinChunkKeys) L = layout_for(ctx, keys = std::max(keys / 2, kMinChunkKeys), nb);
+    if (L.bytes > w.bytes) {
+      if (L.bytes > room) return S615_OK;
+      stage_release(ctx);
+      void* p = nullptr;
+      if (dev_alloc_once(ctx, &p, L.bytes)) return S615_OK;
+      w.p = p;
+      w.bytes = L.bytes;
+    }
+  }
+  if (!w.last) S615_CU(cudaEventCreateWithFlags(&w.last, cudaEventDisableTiming));
+  else S615_CU(cudaStreamWaitEvent(st, w.last, 0));   // the space's last user, on any stream
+  *done = true;
+  StageChunk* chunk = static_cast<StageChunk*>(w.p);
+  char* at = static_cast<char*>(w.p) + (sizeof(StageChunk) + 255) / 256 * 256;
+  auto* first = reinterpret_cast<unsigned long long*>(at);
+  auto* second = reinterpret_cast<unsigned long long*>(at + L.first);
+  const StagePages pages{first, reinterpret_cast<u32*>(first + (size_t)nb * L.pages * kStagePage),
+                         chunk->count[0], nb, L.pages};
+  const u64 chunks = std::max<u64>(1, (u64)(est / (double)keys + 0.999));
+  int s = S615_OK;
+  for (u64 c = 0; c < chunks && !s; ++c) {
+    const u32 lo = (u32)(b->n_main * c / chunks), hi = (u32)(b->n_main * (c + 1) / chunks);
+    if (lo == hi) continue;
+    if (cudaMemsetAsync(chunk, 0, sizeof(StageChunk), st) != cudaSuccess) { s = S615_E_DEVICE; break; }
+    if ((s = launch_stage_peel(ctx, tv, b, flags, st, false, lo, hi, sb, pages, chunk))) break;
+    StageParams P{};
+    P.tv = tv;
+    P.plane = tv.splane;
+    P.sb = sb;
+    P.chunk = chunk;
+    P.first = pages;
+    P.out = StageRuns{second, chunk->count[1], nb, L.entries};
+    if ((s = launch_stage(ctx, k_stage<1>, P, st))) break;
+    P.in = P.out;
+    P.out = StageRuns{first, chunk->count[2], nb, L.entries};
+    if ((s = launch_stage(ctx, k_stage<2>, P, st))) break;
+    P.in = P.out;
+    if ((s = launch_stage(ctx, k_stage_last, P, st))) break;
+    s = launch_stage_peel(ctx, tv, b, flags, st, true, lo, hi, sb, pages, chunk);
+  }
+  cudaEventRecord(w.last, st);
+  return s;
+}
+
+}  // namespace s615

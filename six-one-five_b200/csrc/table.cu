@@ -126,7 +126,8 @@ TableView view_of(const DevTable& t) {
   v.r = t.hdr.r;
   v.layout = (u32)t.layout;
   v.cell_bytes = (u32)t.cell_bytes;
-  v.plane = static_cast<const u32*>(t.d_plane);
+  v.plane = t.plane_staged ? nullptr : static_cast<const u32*>(t.d_plane);
+  v.splane = t.plane_staged ? static_cast<const u32*>(t.d_plane) : nullptr;
   v.plane_bytes = t.plane_bytes;
   v.plane_lb = t.plane_lb;
   v.plane_mask = (u32)((1ull << (1u << t.plane_lb)) - 1);
@@ -158,11 +159,19 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
     const double ps = 3 * read_ps(mb) + cell_ps / (double)(1u << bits);
     if (mb <= kPlaneMaxMB && ps < best) { best = ps; lb = k; }
   }
-  if (lb < 0) return S615_OK;
+  const bool staged = lb < 0;
+  if (staged) {   // 4 bits for the staged probe, when its slices (staged.cuh) fit L2
+    if (t.bytes < ((size_t)1 << 30) || t.hdr.r < 4 || m / 2 / 3 / 16 > kStageSlice) return S615_OK;
+    lb = 2;
+  }
   const u32 per = 32u >> lb;
   const u64 words = (m + per - 1) / per;
   void* p = nullptr;
-  if (dev_alloc(ctx, &p, words * sizeof(u32))) return S615_OK;   // no room: the cells alone
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
+  // no room, or room that a search will want: the cells alone
+  if (staged && 4 * words * sizeof(u32) > free_b) return S615_OK;
+  if (dev_alloc_once(ctx, &p, words * sizeof(u32))) return S615_OK;
   k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
                                                      t.hdr.r, m, (u32)lb, static_cast<u32*>(p), words);
   ctx->launches++;
@@ -175,6 +184,7 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   t.d_plane = p;
   t.plane_bytes = words * sizeof(u32);
   t.plane_lb = (u32)lb;
+  t.plane_staged = staged;
   return S615_OK;
 }
 
