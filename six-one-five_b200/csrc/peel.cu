@@ -544,11 +544,16 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
     if (b->blocks_per_sm && (int)b->blocks_per_sm < per_sm) per_sm = (int)b->blocks_per_sm;
     grid = ctx->num_sms * (per_sm > 0 ? per_sm : 1);
   }
-  // The staged probe's passes deal items out in parts, until each warp has 16 of
-  // them to take or a part is down to 256 keys (its row set-up then shows).
+  // Parts: a launch ends when its last item does, and warps of a large SM group
+  // take theirs slowest (scattered reads are shared per group), so items are
+  // dealt out in parts until each warp has 48 of them to take or a part is down
+  // to 256 keys (its row set-up then shows).  A 50-unit request of the 3.2M band
+  // (6,002 items for 5,920 warps): 2.83 -> 1.65 ms; class-5 band at 1M 8.9 ->
+  // 8.2 ms.  The sharp gate's rows cost more to set up and wait for few probes
+  // (8), and the staged probe's two passes wait for none (16).
   const u64 n_here = n - P.item_lo, warps = (u64)grid * kWarps;
   const double per_item = b->est_keys / (double)std::max<size_t>(b->n_main, 1);
-  while (kMode != kProbe && P.sub_log2 < 4 && (n_here << P.sub_log2) < warps * 16 &&
+  while (P.sub_log2 < 4 && (n_here << P.sub_log2) < warps * (kSharp ? 8 : kMode == kProbe ? 48 : 16) &&
          per_item >= (double)(512u << P.sub_log2))
     ++P.sub_log2;
   const size_t need = ((n_here << P.sub_log2) + kWarps - 1) / kWarps;
