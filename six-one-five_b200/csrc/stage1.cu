@@ -130,28 +130,31 @@ __global__ void k_s1_gather(const DevUnit* units, u32 n, u64* bu) {
 }
 
 int roots_on_device(s615_ctx* ctx, Roots* R) {
-  std::vector<u32> o2, r2, o3, r3, o7, r7;
-  root_csr(2, o2, r2);
-  root_csr(3, o3, r3);
-  root_csr(7, o7, r7);
-  const size_t words = o2.size() + r2.size() + o3.size() + r3.size() + o7.size() + r7.size();
+  // an offset per residue and one, then the units mod 2^6, 3^6, 7^6
+  constexpr size_t n2 = kM2 + 1, u2 = kM2 / 2, n3 = kM3 + 1, u3 = kM3 / 3 * 2, n7 = kM7 + 1,
+                   u7 = kM7 / 7 * 6, words = n2 + u2 + n3 + u3 + n7 + u7;
   if (!ctx->d_roots) {
-    void* p = nullptr;
-    const int s = dev_alloc(ctx, &p, words * sizeof(u32));
-    if (s) return s;
+    std::vector<u32> o2, r2, o3, r3, o7, r7;
+    root_csr(2, o2, r2);
+    root_csr(3, o3, r3);
+    root_csr(7, o7, r7);
     std::vector<u32> all;
     all.reserve(words);
     for (auto* v : {&o2, &r2, &o3, &r3, &o7, &r7}) all.insert(all.end(), v->begin(), v->end());
+    if (all.size() != words) return S615_E_DEVICE;
+    void* p = nullptr;
+    const int s = dev_alloc(ctx, &p, words * sizeof(u32));
+    if (s) return s;
     S615_CU(cudaMemcpy(p, all.data(), words * sizeof(u32), cudaMemcpyHostToDevice));
     ctx->d_roots = static_cast<u32*>(p);
     ctx->roots_bytes = words * sizeof(u32);
   }
   const u32* q = ctx->d_roots;
-  R->off2 = q; q += o2.size();
-  R->r2 = q; q += r2.size();
-  R->off3 = q; q += o3.size();
-  R->r3 = q; q += r3.size();
-  R->off7 = q; q += o7.size();
+  R->off2 = q; q += n2;
+  R->r2 = q; q += u2;
+  R->off3 = q; q += n3;
+  R->r3 = q; q += u3;
+  R->off7 = q; q += n7;
   R->r7 = q;
   R->inv14_3 = inv_pow6_mod(14, kM3);
   R->inv21_2 = inv_pow6_mod(21, kM2);
@@ -197,10 +200,11 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
   }
   S615_CU(cudaMemcpyAsync(d_off, off.data(), nB * 4, cudaMemcpyHostToDevice, st));
   // 2. the batch's unit records and item counts
+  // (the four buffers come from the context's pool, as s615_prepare's do)
   const size_t nu = std::max<size_t>(n_units, 1);
-  if ((s = dev_alloc(ctx, &p, nu * sizeof(DevUnit)))) return s;
+  if ((s = pool_get(ctx, nu * sizeof(DevUnit), &p, &b->units_bytes))) return s;
   b->d_units = static_cast<DevUnit*>(p);
-  b->cap_units = nu;
+  b->cap_units = b->units_bytes / sizeof(DevUnit);
   b->n_units = n_units;
   if ((s = arena_get(ctx, 1, nu * 4 * 2 + 16, &p))) { s615_batch_free(ctx, b.release()); return s; }
   u32* d_ni = static_cast<u32*>(p);
@@ -218,9 +222,9 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
   if (n_items >> 32) { s615_batch_free(ctx, b.release()); return S615_E_ARG; }
   // 3. work items
   const size_t nit = std::max<size_t>(n_items, 1);
-  if ((s = dev_alloc(ctx, &p, nit * sizeof(u64)))) { s615_batch_free(ctx, b.release()); return s; }
+  if ((s = pool_get(ctx, nit * sizeof(u64), &p, &b->items_bytes))) { s615_batch_free(ctx, b.release()); return s; }
   b->d_items = static_cast<u64*>(p);
-  b->cap_items = nit;
+  b->cap_items = b->items_bytes / sizeof(u64);
   b->n_items = n_items;
   b->n_main = n_items;
   if (n_units) {
@@ -230,10 +234,10 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
     S615_CU(cudaGetLastError());
   }
   // 4. counters, cursors, hits
-  if ((s = dev_alloc(ctx, &p, sizeof(Cls5Counters) + 64))) { s615_batch_free(ctx, b.release()); return s; }
+  if ((s = pool_get(ctx, sizeof(Cls5Counters) + 64, &p, &b->ctr_bytes))) { s615_batch_free(ctx, b.release()); return s; }
   b->d_ctr = static_cast<Cls5Counters*>(p);
   b->d_work = reinterpret_cast<u32*>(static_cast<char*>(p) + sizeof(Cls5Counters));
-  if ((s = dev_alloc(ctx, &p, (size_t)(1u << 20) * sizeof(s615_hit)))) {
+  if ((s = pool_get(ctx, (size_t)(1u << 20) * sizeof(s615_hit), &p, &b->hits_bytes))) {
     s615_batch_free(ctx, b.release());
     return s;
   }
