@@ -396,6 +396,7 @@ int s615_close(s615_ctx* ctx) {
   ctx->tables.clear();
   dev_free(ctx, ctx->d_pat, (4 * kPatWords + kTriWords + 2 * kSharpWords) * sizeof(u32));
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
+  if (ctx->aux) cudaStreamDestroy(ctx->aux);
   delete ctx;
   return S615_OK;
 }
@@ -922,6 +923,27 @@ static int pack_units(s615_ctx* ctx, const s615_unit* units, size_t n, DevUnit**
   return S615_OK;
 }
 
+// Items of the second kernel past which their order is made on the device.
+constexpr size_t kOrderOnDevice = 1u << 14;
+
+// The batch's second-kernel items from the host copy into d_items, by chunk.
+static int upload_ordered(s615_ctx* ctx, s615_batch* b) {
+  const size_t n = b->n_items - b->n_main, bytes = n * sizeof(u64);
+  if (!ctx->aux) S615_CU(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+  void *raw = nullptr, *scratch = nullptr;
+  size_t raw_bytes = 0, scratch_bytes = 0;
+  int s = pool_get(ctx, bytes, &raw, &raw_bytes);
+  if (!s) s = pool_get(ctx, order_items_scratch(ctx, n), &scratch, &scratch_bytes);
+  if (!s && cudaMemcpyAsync(raw, b->host_items.get() + b->n_main, bytes, cudaMemcpyHostToDevice,
+                            ctx->aux) != cudaSuccess)
+    s = S615_E_DEVICE;
+  if (!s) s = order_items(ctx, static_cast<const u64*>(raw), b->d_items + b->n_main, n, scratch, ctx->aux);
+  if (cudaStreamSynchronize(ctx->aux) != cudaSuccess && !s) s = S615_E_DEVICE;
+  pool_put(ctx, raw, raw_bytes);
+  pool_put(ctx, scratch, scratch_bytes);
+  return s;
+}
+
 int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   b->n_items = b->n_main = 0;
   DevUnit* du = nullptr;
@@ -1020,9 +1042,13 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
     }
   });
   // heaviest first: a candidate's first rows (smallest d) have the largest T
-  // and windows, so every candidate's chunk 0 goes out before any chunk 1
-  std::stable_sort(items + at[nt], items + total,
-                   [](u64 a, u64 c) { return item_chunk(a) < item_chunk(c); });
+  // and windows, so every candidate's chunk 0 goes out before any chunk 1.  A
+  // long list is put in that order on the device, on its way into place.
+  const size_t n617 = total - at[nt];
+  const bool order_on_device = n617 > kOrderOnDevice;
+  if (!order_on_device)
+    std::stable_sort(items + at[nt], items + total,
+                     [](u64 a, u64 c) { return item_chunk(a) < item_chunk(c); });
   nvtxRangePop();
   NvtxRange upload("upload batch");
   b->n_units = nd;
@@ -1063,9 +1089,10 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   }
   if (nd)
     S615_CU(cudaMemcpy(b->d_units, du, nd * sizeof(DevUnit), cudaMemcpyHostToDevice));
-  if (b->n_items)
-    S615_CU(cudaMemcpy(b->d_items, b->host_items.get(), b->n_items * sizeof(u64), cudaMemcpyHostToDevice));
-  return S615_OK;
+  const size_t n_plain = order_on_device ? b->n_main : b->n_items;
+  if (n_plain)
+    S615_CU(cudaMemcpy(b->d_items, b->host_items.get(), n_plain * sizeof(u64), cudaMemcpyHostToDevice));
+  return order_on_device ? upload_ordered(ctx, b) : S615_OK;
 }
 
 }  // namespace s615
@@ -1135,6 +1162,11 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
     mark_done();
     return s;
   }
+  // The second kernel's items in the host copy's order, which the loop below goes
+  // by (they may have been ordered on the device).
+  if (b->n_items > b->n_main && b->host_items)
+    S615_CU(cudaMemcpyAsync(b->d_items + b->n_main, b->host_items.get() + b->n_main,
+                            (b->n_items - b->n_main) * sizeof(u64), cudaMemcpyHostToDevice, st));
   // Plain form: one unit per launch and a sync after each, like the
   // reference's per-chunk loop.  (cls 7 items go out heaviest first, so a
   // cls 7 unit's items are not contiguous: each run of them is one launch.)

@@ -261,6 +261,7 @@ struct s615_ctx {
   size_t pool_bytes = 0;
   std::mutex pool_mu;
   bool run_busy = false;
+  cudaStream_t aux = nullptr;   // fill_batch's own kernels, beside any run
   s615::StageSpace stage;
   // L2-persisting access windows (cudaDevAttrMaxPersistingL2CacheSize,
   // cudaDevAttrMaxAccessPolicyWindowSize) and the set-aside this context
@@ -350,6 +351,11 @@ int launch_pack(s615_ctx* ctx, const void* d_wide, int cell_bytes, u64 m, u32 r,
 int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u64* d_keys,
                      u64 n_keys, int r, const u64* seeds, int n_seeds, int N, int layout,
                      DevTable* out, u32 shards = 1, u32 shard = 0);
+
+// Orders n work items by ascending chunk field (beyond the first 1,023 values in
+// no order) from `in` to `out`, on the device; see xor_build.cu.
+int order_items(s615_ctx* ctx, const u64* in, u64* out, u64 n, void* scratch, cudaStream_t st);
+size_t order_items_scratch(const s615_ctx* ctx, u64 n);
 
 // Device verifier; see verify.cu.
 int verify_device(s615_ctx* ctx, const s615_unit* units, size_t n_units, const s615_hit* hits,

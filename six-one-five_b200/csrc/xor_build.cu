@@ -119,6 +119,7 @@ __device__ __forceinline__ void block_positions(const bool (&take)[K], unsigned 
 // the 219 ms of the N = 48,000 incidence); runs of 5 to 12 items divide the
 // store requests accordingly.
 constexpr u32 kMaxSlices = 4608;
+constexpr u32 kItemChunks = 1024;   // order_items: chunk fields told apart
 constexpr int kPartThreads = 512;
 constexpr int kPartPer = 16;
 constexpr u32 kTile = kPartThreads * kPartPer;   // items per tile: 64 KB staged
@@ -1311,6 +1312,33 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
   S615_CU(cudaStreamSynchronize(st));
   S615_CU(cudaGetLastError());
   return S615_OK;
+}
+
+namespace {
+// Work items by chunk field (its last slice takes every larger one).
+struct ItemSource {
+  const u64* items;
+  u32 S;
+  static constexpr int kItems = 1;
+  __device__ __forceinline__ void get(u64 t, u64 (&item)[1], u32 (&sl)[1]) const {
+    item[0] = items[t];
+    sl[0] = min(item_chunk(item[0]), S - 1);
+  }
+};
+}  // namespace
+
+// The builder's partition, with chunks for slices: 18 ms of std::stable_sort on
+// the host for 924,000 items of (6,1,7) find4 jobs, 0.1 ms here.
+int order_items(s615_ctx* ctx, const u64* in, u64* out, u64 n, void* scratch, cudaStream_t st) {
+  const u32 G = part_blocks(ctx, n);
+  const PartScratch ps(scratch, G, kItemChunks);
+  const ItemSource src{in, kItemChunks};
+  if (const int s = part_count(ctx, src, 0, n, G, kItemChunks, ps, st)) return s;
+  return part_scatter(ctx, src, 0, n, G, kItemChunks, 0, kItemChunks, ps,
+                      reinterpret_cast<unsigned long long*>(out), st);
+}
+size_t order_items_scratch(const s615_ctx* ctx, u64 n) {
+  return PartScratch::bytes(part_blocks(ctx, n), kItemChunks);
 }
 
 S615_CHECK_TAKE_DEFINE(check_take_xor_build)
