@@ -63,8 +63,9 @@ inline u64 capacity_for(u64 n) {
 }
 
 // Reciprocal for the exact 64-bit remainder used by every probe: for
-// block >= 2, q = umulhi(h, floor((2^64-1)/block)) undershoots h/block by at
-// most 2, so two conditional subtractions give h % block exactly.
+// block >= 2, recip = floor((2^64-1)/block) >= 2^64/block - 1, so h * recip / 2^64
+// > h/block - 1 and q = umulhi(h, recip) undershoots floor(h/block) by at most 1:
+// one conditional subtraction gives h % block exactly.
 inline u64 mod_recip(u64 block) { return block >= 2 ? (~0ULL) / block : 0; }
 
 S615_HD u64 mulhi64(u64 a, u64 b) {
@@ -77,7 +78,6 @@ S615_HD u64 mulhi64(u64 a, u64 b) {
 
 S615_HD u64 fast_mod(u64 h, u64 block, u64 recip) {
   u64 r = h - mulhi64(h, recip) * block;
-  if (r >= block) r -= block;
   if (r >= block) r -= block;
   return r;
 }

@@ -90,12 +90,10 @@ __device__ __forceinline__ u64 hash_of_word(u64 g) {
   return T == 0 ? g : unmix64(g) ^ (T == 1 ? kPhi : kSalt2);
 }
 
-// g = q * block + off (the exact quotient: mulhi undershoots it by at most 2).
-// (block < 2^32: the remainder before the corrections is below 3 * block.)
+// g = q * block + off (the exact quotient: mulhi undershoots it by at most 1).
 __device__ __forceinline__ void split_word(u64 g, u32 block, u64 recip, u64& q, u32& off) {
   q = mulhi64(g, recip);
   u64 r = g - q * block;
-  if (r >= block) { r -= block; ++q; }
   if (r >= block) { r -= block; ++q; }
   off = (u32)r;
 }

@@ -137,8 +137,7 @@ struct KeySource {
   __device__ __forceinline__ u64 key(u64 t) const {
     if (!vals) return keys[t];
     const u64 len = nv + 1;
-    u64 p = mulhi64(t, row_recip), q = t - p * len;   // p is at most 2 short
-    if (q >= len) { q -= len; ++p; }
+    u64 p = mulhi64(t, row_recip), q = t - p * len;   // p is at most 1 short
     if (q >= len) { q -= len; ++p; }
     const u64 first = nv - p;
     const u64 a = q < first ? p : nv - 1 - p;
