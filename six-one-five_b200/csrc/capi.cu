@@ -397,6 +397,7 @@ int s615_close(s615_ctx* ctx) {
   dev_free(ctx, ctx->d_pat, (4 * kPatWords + kTriWords + 2 * kSharpWords) * sizeof(u32));
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
+  if (ctx->last_run) cudaEventDestroy(ctx->last_run);
   delete ctx;
   return S615_OK;
 }
@@ -886,14 +887,6 @@ static void run_threads(size_t nt, F&& work) {
   for (auto& x : th) x.join();
 }
 
-// About how many of a class 2-5 unit's points pass the gate (2.7% of the R > 0
-// points; a find3 row's window is about 0.15 lim long).
-static double est_keys(const DevUnit& d) {
-  if (d.cls == kClsJobRow) return d.w ? 0.03 : 0.004 * d.lim;
-  const double rows = (double)d.fmax1 / d.mod1 * d.nres1;
-  return rows * (d.cls == 5 ? 0.0243 * d.nres2 * d.fmax2 / 64 : 0.0043 * d.lim);
-}
-
 // make_dev_unit over every unit (on several host threads for large batches),
 // the kept records compacted in unit order.  Returns the error of the
 // lowest-index unit that has one, as a sequential pass would.
@@ -923,6 +916,134 @@ static int pack_units(s615_ctx* ctx, const s615_unit* units, size_t n, DevUnit**
   return S615_OK;
 }
 
+// Room for n_units records, n_items items, the counters and the hits (a reused
+// batch's buffers only grow).
+static int batch_buffers(s615_ctx* ctx, s615_batch* b, size_t n_units, size_t n_items) {
+  int s = 0;
+  void* p = nullptr;
+  size_t got = 0;
+  if (!b->d_units || n_units > b->cap_units) {
+    pool_put(ctx, b->d_units, b->units_bytes);
+    b->d_units = nullptr;
+    b->cap_units = b->units_bytes = 0;
+    if ((s = pool_get(ctx, std::max<size_t>(n_units, 1) * sizeof(DevUnit), &p, &got))) return s;
+    b->d_units = static_cast<DevUnit*>(p);
+    b->units_bytes = got;
+    b->cap_units = got / sizeof(DevUnit);
+  }
+  if (!b->d_items || n_items > b->cap_items) {
+    pool_put(ctx, b->d_items, b->items_bytes);
+    b->d_items = nullptr;
+    b->cap_items = b->items_bytes = 0;
+    if ((s = pool_get(ctx, std::max<size_t>(n_items, 1) * sizeof(u64), &p, &got))) return s;
+    b->d_items = static_cast<u64*>(p);
+    b->items_bytes = got;
+    b->cap_items = got / sizeof(u64);
+  }
+  if (!b->d_ctr) {
+    if ((s = pool_get(ctx, sizeof(Cls5Counters) + 64, &p, &got))) return s;
+    b->d_ctr = static_cast<Cls5Counters*>(p);
+    b->d_work = reinterpret_cast<u32*>(static_cast<char*>(p) + sizeof(Cls5Counters));
+    b->ctr_bytes = got;
+  }
+  if (!b->d_hits) {
+    if ((s = pool_get(ctx, (size_t)(1u << 20) * sizeof(s615_hit), &p, &got))) return s;
+    b->d_hits = static_cast<s615_hit*>(p);
+    b->hit_cap = 1u << 20;
+    b->hits_bytes = got;
+  }
+  return S615_OK;
+}
+
+// Job rows per item: up to 64, fewer when the batch is small, so that its
+// items still fill the GPU (about 64 warps per SM).
+static u32 job_rows_for(const s615_ctx* ctx, size_t n) {
+  u32 job_rows = 8;
+  while (job_rows < kJobRows && (u64)job_rows * ctx->num_sms * 64 < n) job_rows *= 2;
+  return job_rows;
+}
+static u32 tune_bucket(size_t n) {
+  u32 bucket = 0;
+  while (bucket < 39 && (2ull << bucket) <= n) ++bucket;
+  return bucket;
+}
+
+// Whether kernels of fill_batch would start at once.  Beside a running batch,
+// whose persistent grid fills the SMs, they would wait for it to end, and a
+// caller (or the serving loop) that prepares a batch while another runs would
+// lose that overlap: then the host does the work.
+static bool device_idle(s615_ctx* ctx) {
+  if (ctx->server) return false;
+  if (!ctx->last_run) return true;
+  const cudaError_t e = cudaEventQuery(ctx->last_run);
+  if (e != cudaSuccess && e != cudaErrorNotReady) cudaGetLastError();
+  return e == cudaSuccess;
+}
+
+// fill_batch on the device (pack.cu).  *done = false: the batch holds units of
+// other classes, is too small for the two extra round trips to pay, or the
+// device is busy or short of memory.
+constexpr size_t kDeviceFill = 128;
+static int fill_on_device(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b, bool* done) {
+  *done = false;
+  if (n < kDeviceFill || !device_idle(ctx)) return S615_OK;
+  // the caller's records through pinned memory, looked over on the way
+  auto* stage = static_cast<s615_unit*>(stage_get(ctx->unit_stage, n * sizeof(s615_unit)));
+  if (!stage) return S615_E_OOM;
+  const size_t nt = host_threads(n);
+  std::vector<char> other(nt, 0);
+  run_threads(nt, [&](size_t t) {
+    for (size_t i = n * t / nt, hi = n * (t + 1) / nt; i < hi; ++i) {
+      if (units[i].cls < 2 || units[i].cls > 5) { other[t] = 1; return; }
+      stage[i] = units[i];
+    }
+  });
+  for (char o : other)
+    if (o) return S615_OK;
+  if (!ctx->aux) S615_CU(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+  const u32 job_rows = job_rows_for(ctx, n);
+  void *raw = nullptr, *tot = nullptr;
+  size_t raw_bytes = 0, tot_bytes = 0;
+  FillTotals h{};
+  int s = batch_buffers(ctx, b, n, 0);
+  if (!s) s = pool_get(ctx, n * sizeof(s615_unit), &raw, &raw_bytes);
+  if (!s) s = pool_get(ctx, sizeof(FillTotals), &tot, &tot_bytes);
+  auto cu = [&](cudaError_t e) { if (!s && e != cudaSuccess) s = cuda_status(e); };
+  auto* d_raw = static_cast<const s615_unit*>(raw);
+  auto* d_tot = static_cast<FillTotals*>(tot);
+  if (!s) cu(cudaMemcpyAsync(raw, stage, n * sizeof(s615_unit), cudaMemcpyHostToDevice, ctx->aux));
+  if (!s) s = launch_pack(ctx, d_raw, (u32)n, job_rows, b->d_units, d_tot, ctx->aux);
+  if (!s) cu(cudaMemcpyAsync(&h, tot, sizeof h, cudaMemcpyDeviceToHost, ctx->aux));
+  if (!s) cu(cudaStreamSynchronize(ctx->aux));
+  if (!s && h.bad) s = S615_E_FORMAT;
+  if (!s) {
+    // rows per item by fill_batch's rule
+    const auto& tuned = ctx->tune[tune_bucket(n)];
+    b->blocks_per_sm = ctx->force_bps ? ctx->force_bps : tuned.blocks_per_sm;
+    const u32 set = ctx->force_rows ? ctx->force_rows : tuned.item_rows;
+    int q = 0;
+    if (set) q = set >= 64 ? 0 : set >= 32 ? 1 : 2;
+    else while (q < 2 && h.items5[q] + h.items234[q] < (u64)ctx->num_sms * 40) ++q;
+    b->item_rows = kItemRows >> q;
+    b->parts3 = !set && q == 2 ? 4u : 1u;
+    b->n_units = n;
+    b->n_items = b->n_main = h.items5[q] + h.items234[q] * b->parts3 + h.jobs;
+    b->est_keys = h.keys;
+    b->host_items_valid = false;
+    b->h2d_bytes = n * sizeof(s615_unit);
+    s = batch_buffers(ctx, b, n, b->n_items);
+    if (!s && b->n_items)
+      s = launch_items(ctx, d_raw, b->d_units, (u32)n, job_rows, b->item_rows, b->parts3, b->d_items,
+                       b->n_items, d_tot, ctx->aux);
+  }
+  if (cudaStreamSynchronize(ctx->aux) != cudaSuccess && !s) s = S615_E_DEVICE;
+  pool_put(ctx, raw, raw_bytes);
+  pool_put(ctx, tot, tot_bytes);
+  if (s == S615_E_OOM) return S615_OK;   // the host's way needs less
+  *done = true;
+  return s;
+}
+
 // Items of the second kernel past which their order is made on the device.
 constexpr size_t kOrderOnDevice = 1u << 14;
 
@@ -946,23 +1067,28 @@ static int upload_ordered(s615_ctx* ctx, s615_batch* b) {
 
 int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   b->n_items = b->n_main = 0;
+  {
+    NvtxRange nvtx("pack on the device");
+    bool done = false;
+    const int s = fill_on_device(ctx, units, n, b, &done);
+    if (s || done) {
+      if (s) b->n_items = b->n_main = 0;
+      return s;
+    }
+  }
+  b->host_items_valid = true;
   DevUnit* du = nullptr;
   size_t nd = 0;
   {
     NvtxRange nvtx("pack units");
     if (const int s = pack_units(ctx, units, n, &du, &nd)) return s;
   }
-  // Job rows per item: up to 64, fewer when the batch is small, so that its
-  // items still fill the GPU (about 64 warps per SM).
-  u32 job_rows = 8;
-  while (job_rows < kJobRows && (u64)job_rows * ctx->num_sms * 64 < nd) job_rows *= 2;
+  const u32 job_rows = job_rows_for(ctx, nd);
   // Rows per class 2-5 item: 64, or 32 / 16 when a batch would otherwise
   // have fewer items than about 40 warps per SM (a small serving batch).
   const u64 want_items = (u64)ctx->num_sms * 40;
   u32 unit_rows = kItemRows;
-  u32 bucket = 0;
-  while (bucket < 39 && (2ull << bucket) <= n) ++bucket;
-  const auto& tuned = ctx->tune[bucket];
+  const auto& tuned = ctx->tune[tune_bucket(n)];
   b->blocks_per_sm = ctx->force_bps ? ctx->force_bps : tuned.blocks_per_sm;
   if (ctx->force_rows || tuned.item_rows) {
     unit_rows = ctx->force_rows ? ctx->force_rows : tuned.item_rows;
@@ -1010,7 +1136,7 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
       const DevUnit& d = du[k];
       if (d.cls == 0) continue;   // dropped
       if (second(d)) unit_items(d, (u32)k, c, job_rows, unit_rows, b->parts3);
-      else unit_items(d, (u32)k, m, job_rows, unit_rows, b->parts3), keys += est_keys(d);
+      else unit_items(d, (u32)k, m, job_rows, unit_rows, b->parts3), keys += unit_keys(d);
     }
     cnt_main[t] = m.n;
     cnt_617[t] = c.n;
@@ -1045,7 +1171,7 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   // and windows, so every candidate's chunk 0 goes out before any chunk 1.  A
   // long list is put in that order on the device, on its way into place.
   const size_t n617 = total - at[nt];
-  const bool order_on_device = n617 > kOrderOnDevice;
+  const bool order_on_device = n617 > kOrderOnDevice && device_idle(ctx);
   if (!order_on_device)
     std::stable_sort(items + at[nt], items + total,
                      [](u64 a, u64 c) { return item_chunk(a) < item_chunk(c); });
@@ -1054,39 +1180,8 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   b->n_units = nd;
   b->n_main = at[nt];
   b->n_items = total;
-  int s = 0;
-  void* p = nullptr;
-  size_t got = 0;
-  if (!b->d_units || nd > b->cap_units) {
-    pool_put(ctx, b->d_units, b->units_bytes);
-    b->d_units = nullptr;
-    b->cap_units = b->units_bytes = 0;
-    if ((s = pool_get(ctx, std::max<size_t>(nd, 1) * sizeof(DevUnit), &p, &got))) return s;
-    b->d_units = static_cast<DevUnit*>(p);
-    b->units_bytes = got;
-    b->cap_units = got / sizeof(DevUnit);
-  }
-  if (!b->d_items || b->n_items > b->cap_items) {
-    pool_put(ctx, b->d_items, b->items_bytes);
-    b->d_items = nullptr;
-    b->cap_items = b->items_bytes = 0;
-    if ((s = pool_get(ctx, std::max<size_t>(b->n_items, 1) * sizeof(u64), &p, &got))) return s;
-    b->d_items = static_cast<u64*>(p);
-    b->items_bytes = got;
-    b->cap_items = got / sizeof(u64);
-  }
-  if (!b->d_ctr) {
-    if ((s = pool_get(ctx, sizeof(Cls5Counters) + 64, &p, &got))) return s;
-    b->d_ctr = static_cast<Cls5Counters*>(p);
-    b->d_work = reinterpret_cast<u32*>(static_cast<char*>(p) + sizeof(Cls5Counters));
-    b->ctr_bytes = got;
-  }
-  if (!b->d_hits) {
-    if ((s = pool_get(ctx, (size_t)(1u << 20) * sizeof(s615_hit), &p, &got))) return s;
-    b->d_hits = static_cast<s615_hit*>(p);
-    b->hit_cap = 1u << 20;
-    b->hits_bytes = got;
-  }
+  b->h2d_bytes = nd * sizeof(DevUnit) + total * sizeof(u64);
+  if (const int s = batch_buffers(ctx, b, nd, total)) return s;
   if (nd)
     S615_CU(cudaMemcpy(b->d_units, du, nd * sizeof(DevUnit), cudaMemcpyHostToDevice));
   const size_t n_plain = order_on_device ? b->n_main : b->n_items;
@@ -1118,7 +1213,7 @@ int s615_batch_size(const s615_batch* b, size_t* n_units, size_t* n_items, size_
   if (!b) return S615_E_ARG;
   if (n_units) *n_units = b->n_units;
   if (n_items) *n_items = b->n_items;
-  if (h2d_bytes) *h2d_bytes = b->n_units * sizeof(DevUnit) + b->n_items * sizeof(u64);
+  if (h2d_bytes) *h2d_bytes = b->h2d_bytes;
   return S615_OK;
 }
 
@@ -1153,6 +1248,16 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
       b->done = nullptr;
     }
     if (b->done) cudaEventRecord(b->done, st);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return;
+    }
+    if (!ctx->last_run && cudaEventCreateWithFlags(&ctx->last_run, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      ctx->last_run = nullptr;
+    }
+    if (ctx->last_run) cudaEventRecord(ctx->last_run, st);
   };
   S615_CU(cudaMemsetAsync(b->d_ctr, 0, sizeof(Cls5Counters) + 64, st));
   if (!(flags & S615_F_PLAIN)) {
@@ -1162,9 +1267,17 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
     mark_done();
     return s;
   }
-  // The second kernel's items in the host copy's order, which the loop below goes
-  // by (they may have been ordered on the device).
-  if (b->n_items > b->n_main && b->host_items)
+  // The loop below goes by the host copy of the items: the ones made on the device
+  // are fetched, and the second kernel's put in its order (they may have been
+  // ordered on the device).
+  if (!b->host_items_valid && b->n_items) {
+    b->host_items.reset(new (std::nothrow) u64[b->n_items]);
+    b->host_items_cap = b->host_items ? b->n_items : 0;
+    if (!b->host_items) return S615_E_OOM;
+    S615_CU(cudaMemcpy(b->host_items.get(), b->d_items, b->n_items * sizeof(u64), cudaMemcpyDeviceToHost));
+    b->host_items_valid = true;
+  }
+  if (b->n_items > b->n_main)
     S615_CU(cudaMemcpyAsync(b->d_items + b->n_main, b->host_items.get() + b->n_main,
                             (b->n_items - b->n_main) * sizeof(u64), cudaMemcpyHostToDevice, st));
   // Plain form: one unit per launch and a sync after each, like the

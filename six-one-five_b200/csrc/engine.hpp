@@ -202,6 +202,8 @@ struct s615_batch {
   // place by the fill's threads
   std::unique_ptr<s615::u64[]> host_items;
   size_t host_items_cap = 0;
+  bool host_items_valid = false;   // false: made on the device, not copied back
+  size_t h2d_bytes = 0;            // what the last fill copied to the device
 };
 
 namespace s615 {
@@ -261,7 +263,8 @@ struct s615_ctx {
   size_t pool_bytes = 0;
   std::mutex pool_mu;
   bool run_busy = false;
-  cudaStream_t aux = nullptr;   // fill_batch's own kernels, beside any run
+  cudaStream_t aux = nullptr;   // fill_batch's own kernels
+  cudaEvent_t last_run = nullptr;   // after the context's latest s615_run_batch
   s615::StageSpace stage;
   // L2-persisting access windows (cudaDevAttrMaxPersistingL2CacheSize,
   // cudaDevAttrMaxAccessPolicyWindowSize) and the set-aside this context
@@ -356,6 +359,26 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
 // no order) from `in` to `out`, on the device; see xor_build.cu.
 int order_items(s615_ctx* ctx, const u64* in, u64* out, u64 n, void* scratch, cudaStream_t st);
 size_t order_items_scratch(const s615_ctx* ctx, u64 n);
+
+// About how many of a class 2-5 unit's points pass the gate (2.7% of the R > 0
+// points; a find3 row's window is about 0.15 lim long).
+S615_HD double unit_keys(const DevUnit& d) {
+  if (d.cls == kClsJobRow) return d.w ? 0.03 : 0.004 * d.lim;
+  const double rows = (double)d.fmax1 / d.mod1 * d.nres1;
+  return rows * (d.cls == 5 ? 0.0243 * d.nres2 * d.fmax2 / 64 : 0.0043 * d.lim);
+}
+
+// Unit records and work items of classes 2-5 made on the device (pack.cu).
+struct FillTotals {
+  unsigned long long items5[3], items234[3];   // row chunks of 64, 32, 16 rows
+  unsigned long long jobs, placed;             // job items; items written
+  double keys;
+  u32 bad, pad;                                // a unit was refused
+};
+int launch_pack(s615_ctx* ctx, const s615_unit* d_raw, u32 n, u32 job_rows, DevUnit* units,
+                FillTotals* tot, cudaStream_t st);
+int launch_items(s615_ctx* ctx, const s615_unit* d_raw, const DevUnit* units, u32 n, u32 job_rows,
+                 u32 rows, u32 parts3, u64* items, u64 n_items, FillTotals* tot, cudaStream_t st);
 
 // Device verifier; see verify.cu.
 int verify_device(s615_ctx* ctx, const s615_unit* units, size_t n_units, const s615_hit* hits,

@@ -17,24 +17,15 @@
 #include <numeric>
 #include <vector>
 
-#include "engine.hpp"
+#include "pack.cuh"
 
 namespace s615 {
 
 namespace {
 
-constexpr u32 kM2 = 64, kM3 = 729, kM7 = 117649;
+constexpr u32 kM2 = kRootM2, kM3 = kRootM3, kM7 = kRootM7;
 
-struct Roots {                 // CSR root lists, offsets then roots, per modulus
-  const u32 *off2, *r2, *off3, *r3, *off7, *r7;
-  u32 inv14_3, inv21_2;        // (14^6)^-1 mod 3^6, (21^6)^-1 mod 2^6
-};
-
-__device__ __forceinline__ u32 pow6_mod(u64 x, u32 m) {
-  x %= m;
-  const u64 x2 = x * x % m, x3 = x2 * x % m;
-  return (u32)(x3 * x3 % m);
-}
+__device__ __forceinline__ u32 pow6_mod(u64 x, u32 m) { return pow6_mod_u32(x, m); }
 
 __device__ __forceinline__ bool eligible(u64 B) { return B > 1 && (B & 1) && B % 3 && B % 7; }
 
@@ -129,6 +120,8 @@ __global__ void k_s1_gather(const DevUnit* units, u32 n, u64* bu) {
   if (k < n) { bu[2 * k] = units[k].B; bu[2 * k + 1] = units[k].u; }
 }
 
+}  // namespace
+
 int roots_on_device(s615_ctx* ctx, Roots* R) {
   // an offset per residue and one, then the units mod 2^6, 3^6, 7^6
   constexpr size_t n2 = kM2 + 1, u2 = kM2 / 2, n3 = kM3 + 1, u3 = kM3 / 3 * 2, n7 = kM7 + 1,
@@ -158,10 +151,11 @@ int roots_on_device(s615_ctx* ctx, Roots* R) {
   R->r7 = q;
   R->inv14_3 = inv_pow6_mod(14, kM3);
   R->inv21_2 = inv_pow6_mod(21, kM2);
+  R->inv7_2 = inv_pow6_mod(7, kM2);
+  R->inv7_3 = inv_pow6_mod(7, kM3);
+  R->inv64_3 = inv_pow6_mod(2, kM3);   // 64 = 2^6
   return S615_OK;
 }
-
-}  // namespace
 
 }  // namespace s615
 
