@@ -8,9 +8,9 @@
 //   cls 7  : a,b <= N and a^6+b^6+c3^6+c4^6 == T       (solve_617_v1.cu:1083-1088)
 // The surviving set is exactly {(c1,c2): c1 <= c2 <= cmax, c1^6 + c2^6 = S}
 // with S the hit's exact remainder and cmax = min(N, lim), min(N, c3) or N; this
-// kernel enumerates it directly: one warp per hit, the c1 range
-// [1, (S/2)^(1/6)] split into 32 segments, each walked with the two-pointer
-// rule (c1 up, c2 down).  Identity, term and gcd checks run on the host.
+// kernel enumerates it directly: one warp per hit, or up to 64 when there are few
+// hits, the c1 range [1, (S/2)^(1/6)] split into a segment per lane, each walked
+// with the two-pointer rule (c1 up, c2 down).  Identity, term and gcd checks run on the host.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,12 +28,12 @@ namespace {
 struct PairOut { u32 hit, c1, c2, pad; };
 
 __global__ void k_verify(const DevUnit* __restrict__ units, const s615_hit* __restrict__ hits,
-                         u32 n_hits, u32 N, u64 inv_lo, u64 inv_hi, PairOut* out, u32 cap,
+                         u32 n_hits, u32 N, u64 inv_lo, u64 inv_hi, u32 parts, PairOut* out, u32 cap,
                          u32* n_out) {
-  const u32 lane = threadIdx.x & 31;
-  const u32 warps = (gridDim.x * blockDim.x) >> 5;
+  const u32 warps = (gridDim.x * blockDim.x) >> 5, lanes = 32 * parts;
   const u128 inv21 = ((u128)inv_hi << 64) | inv_lo;
-  for (u32 hi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; hi < n_hits; hi += warps) {
+  for (u64 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (u64)n_hits * parts; w += warps) {
+    const u32 hi = (u32)(w / parts), lane = (u32)(w % parts) * 32 + (threadIdx.x & 31);
     const s615_hit H = hits[hi];
     const DevUnit& U = units[H.unit];
     const u128 base = ((u128)U.base_hi << 64) | U.base_lo;
@@ -75,7 +75,7 @@ __global__ void k_verify(const DevUnit* __restrict__ units, const s615_hit* __re
     }
     const u32 c1max = iroot6_u128(S >> 1);
     if (c1max == 0) continue;
-    const u32 seg = (c1max + 31) / 32;
+    const u32 seg = (c1max + lanes - 1) / lanes;
     u32 c1 = 1 + lane * seg;
     const u32 end = min(c1max, c1 + seg - 1);
     if (c1 > c1max) continue;
@@ -139,11 +139,14 @@ int verify_device(s615_ctx* ctx, const s615_unit* units, size_t n_units, const s
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_h, kh.data(), bh, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_n, 0, 16, st);
     if (e == cudaSuccess) {
-      const u32 blocks = (u32)std::min<size_t>((n_hits + 7) / 8, (size_t)ctx->num_sms * 32);
+      // few hits: up to 64 warps for each, so that the walk over a wide c1 range is
+      // not one warp's serial chain
+      const u32 parts = (u32)std::max<size_t>(1, std::min<size_t>(64, (size_t)ctx->num_sms * 16 / n_hits));
+      const u32 blocks = (u32)std::min<size_t>((n_hits * parts + 7) / 8, (size_t)ctx->num_sms * 32);
       k_verify<<<blocks, 256, 0, st>>>(static_cast<const DevUnit*>(d_u),
                                        static_cast<const s615_hit*>(d_h), (u32)n_hits, (u32)N,
-                                       (u64)inv, (u64)(inv >> 64), static_cast<PairOut*>(d_p), pcap,
-                                       static_cast<u32*>(d_n));
+                                       (u64)inv, (u64)(inv >> 64), parts, static_cast<PairOut*>(d_p),
+                                       pcap, static_cast<u32*>(d_n));
       ctx->launches++;
       e = cudaGetLastError();
     }
