@@ -530,6 +530,25 @@ struct ClaimList {
   }
 };
 
+// Rounds of few candidates go out kRounds at a time, each reading its sizes from
+// here: round j of a batch has candidates [0, ncand[j]) and claims the list's
+// entries [end[j], end[j + 1]).  A round whose candidates overflowed their list,
+// and those after it, do nothing.  With the host waiting for the sizes twice in
+// every round, a round took at least 70 us: building N = 1,500 took 7.0 ms,
+// 6,000 11.6 and 16,000 52.0; in batches of 8 it takes 4.5, 9.5 and 50.1.  A
+// batch's grids are for its first round's candidates and half as many again
+// (the kernels stride), so a round with none left costs an empty launch.
+constexpr int kRounds = 8;
+struct PeelState {
+  unsigned long long norder;               // claimed cells so far
+  unsigned long long ncand[kRounds + 1], end[kRounds + 1];
+  u32 over[kRounds + 2];
+};
+// Candidates up to which rounds are batched: 2 million take 0.27 ms, so above
+// it the two waits are less than a fifth of a round, and a batch that a large
+// round shrinks in would launch grids far too wide.
+constexpr u64 kBatchCand = 1ull << 21;
+
 // Claims among the candidate cells [0, ncand), or among every cell when the
 // candidate list is null: a count-1 cell claims its key unless a lower cell of
 // the key has count 1 too.  A candidate costs a chain of scattered reads (its
@@ -538,7 +557,9 @@ struct ClaimList {
 constexpr int kClaimPer = 4;
 __global__ void k_claim_list(CellList cand, u64 ncand, const unsigned long long* __restrict__ W,
                              const u64* __restrict__ keys, u64 seed, u64 block, u64 recip,
-                             ClaimList out, unsigned long long* n_order, u64 order_cap, u32* over) {
+                             ClaimList out, unsigned long long* n_order, u64 order_cap, u32* over,
+                             const PeelState* ps, int j) {
+  if (ps) ncand = ps->over[j] ? 0 : ps->ncand[j];   // round j of a batch
   const u64 span = (u64)blockDim.x * kClaimPer;
   for (u64 base = blockIdx.x * span; base < ncand; base += (u64)gridDim.x * span) {
     bool claim[kClaimPer];
@@ -590,7 +611,14 @@ constexpr int kApplyPer = 4;
 
 __global__ void k_apply_list(ClaimList in, u64 L, unsigned long long* W,
                              const u64* __restrict__ keys, u64 seed, u64 block, u64 recip,
-                             CellList next, unsigned long long* n_next, u64 next_cap, u32* over) {
+                             CellList next, unsigned long long* n_next, u64 next_cap, u32* over,
+                             PeelState* ps, int j) {
+  if (ps) {   // round j of a batch: what its claim appended
+    const u64 from = ps->end[j], to = ps->norder;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ps->end[j + 1] = to;
+    in = in.at(from);
+    L = to - from;
+  }
   const u64 span = (u64)blockDim.x * kApplyPer;
   for (u64 base = blockIdx.x * span; base < L; base += (u64)gridDim.x * span) {
     bool to[2 * kApplyPer];
@@ -1074,14 +1102,15 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     front.release();
     lists = false;
   }
-  if ((s = scratch.alloc(64))) return s;
+  if ((s = scratch.alloc(64 + sizeof(PeelState)))) return s;
   auto* W = static_cast<unsigned long long*>(cells.p);
   const u64* K = static_cast<const u64*>(keys.p);
-  // scratch: [0] max count, [4] list overflow, [8] n_order / n_claimed, [16] n_next
+  // scratch: [0] max count, [4] list overflow, [8] n_claimed, [16] n_next, then the peel's state
   u32* d_max = static_cast<u32*>(scratch.p);
   u32* d_lover = reinterpret_cast<u32*>(static_cast<char*>(scratch.p) + 4);
   auto* d_norder = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch.p) + 8);
   auto* d_nnext = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch.p) + 16);
+  auto* d_peel = reinterpret_cast<PeelState*>(static_cast<char*>(scratch.p) + 64);
   const int g = grid_for(ctx, m, 256);
   // Entry buffers of the binned incidence: all 3n updates when HBM allows,
   // else chunks of keys; with no room for a useful chunk the incidence adds
@@ -1149,7 +1178,7 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
     const u64 seed = seeds[si];
     S615_CU(cudaMemsetAsync(W, 0, m * sizeof(u64), st));
     if (!lists) S615_CU(cudaMemsetAsync(rounds.p, 0, m * sizeof(u16), st));
-    S615_CU(cudaMemsetAsync(scratch.p, 0, 64, st));
+    S615_CU(cudaMemsetAsync(scratch.p, 0, 64 + sizeof(PeelState), st));
     if (ent_cap) {
       if ((s = incidence_binned(ctx, K, n, seed, m, block, recip,
                                 static_cast<unsigned long long*>(ent.p), ent_cap, W, bins.p, st)))
@@ -1177,39 +1206,79 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
       CellList cand{nullptr, nullptr};   // round 1 scans every cell
       int cur = 0;
       // S615_TRACE: per round, the candidates, the keys claimed and the host
-      // time of its claim and apply (each ends in a sync here anyway)
+      // time of its claim and apply (each ends in a sync here anyway; a batch's
+      // time is spread evenly over its rounds, as apply)
       using TClock = std::chrono::steady_clock;
       const auto ms_since = [](TClock::time_point a) {
         return std::chrono::duration<double, std::milli>(TClock::now() - a).count();
       };
       std::vector<std::array<double, 4>> rounds_trace;
+      bool over = false;   // the candidates of the next round overflowed their list
       while (off.size() <= 0xFFFE) {
         const auto t_claim = TClock::now();
-        k_claim_list<<<blocks_for(ncand, 256 * kClaimPer), 256, 0, st>>>(
-            cand, ncand, W, K, seed, block, recip, claim_list, d_norder, n, d_lover);
-        ctx->launches++;
-        unsigned long long h_n[2] = {0, 0};
-        u32 h_lover = 0;
-        S615_CU(cudaMemcpyAsync(&h_n[0], d_norder, 8, cudaMemcpyDeviceToHost, st));
-        S615_CU(cudaStreamSynchronize(st));
-        const u64 L = h_n[0] - total;
-        const double claim_ms = trace.on ? ms_since(t_claim) : 0.0;
-        const auto t_apply = TClock::now();
-        if (L == 0) break;
-        S615_CU(cudaMemsetAsync(d_nnext, 0, 8, st));
-        S615_CU(cudaMemsetAsync(d_lover, 0, 4, st));
-        k_apply_list<<<blocks_for(L, 256 * kApplyPer), 256, 0, st>>>(
-            claim_list.at(total), L, W, K, seed, block, recip, fr[cur ^ 1], d_nnext, fcap, d_lover);
-        ctx->launches++;
-        S615_CU(cudaGetLastError());
-        S615_CU(cudaMemcpyAsync(&h_n[1], d_nnext, 8, cudaMemcpyDeviceToHost, st));
-        S615_CU(cudaMemcpyAsync(&h_lover, d_lover, 4, cudaMemcpyDeviceToHost, st));
-        S615_CU(cudaStreamSynchronize(st));
-        if (trace.on) rounds_trace.push_back({(double)ncand, (double)L, claim_ms, ms_since(t_apply)});
-        total += L;
-        off.push_back(total);
-        cur ^= 1;
-        if (h_lover) {   // candidates overflowed: the next round scans every cell
+        PeelState h{};
+        if (cand.off && ncand <= kBatchCand && off.size() + kRounds <= 0xFFFE) {
+          // a batch of rounds; sizes on the device, the grids for half as many again
+          h.norder = h.end[0] = total;
+          h.ncand[0] = ncand;
+          S615_CU(cudaMemcpyAsync(d_peel, &h, sizeof h, cudaMemcpyHostToDevice, st));
+          const u64 grid_for_n = ncand + ncand / 2;
+          for (int j = 0; j < kRounds; ++j) {
+            k_claim_list<<<blocks_for(grid_for_n, 256 * kClaimPer), 256, 0, st>>>(
+                fr[cur ^ (j & 1)], 0, W, K, seed, block, recip, claim_list, &d_peel->norder, n,
+                d_lover, d_peel, j);
+            k_apply_list<<<blocks_for(grid_for_n, 256 * kApplyPer), 256, 0, st>>>(
+                claim_list, 0, W, K, seed, block, recip, fr[cur ^ (j & 1) ^ 1], &d_peel->ncand[j + 1],
+                fcap, &d_peel->over[j + 1], d_peel, j);
+            ctx->launches += 2;
+          }
+          S615_CU(cudaGetLastError());
+          S615_CU(cudaMemcpyAsync(&h, d_peel, sizeof h, cudaMemcpyDeviceToHost, st));
+          S615_CU(cudaStreamSynchronize(st));
+          bool more = true;
+          for (int j = 0; j < kRounds && more; ++j) {
+            const u64 L = h.end[j + 1] - h.end[j];
+            if (trace.on) rounds_trace.push_back({(double)h.ncand[j], (double)L, 0, ms_since(t_claim) / kRounds});
+            if (L == 0) { more = false; break; }
+            total += L;
+            off.push_back(total);
+            cur ^= 1;
+            ncand = h.ncand[j + 1];
+            over = h.over[j + 1] != 0;
+            more = ncand != 0 || over;
+            if (over) break;
+          }
+          if (!more) break;
+        } else {
+          k_claim_list<<<blocks_for(ncand, 256 * kClaimPer), 256, 0, st>>>(
+              cand, ncand, W, K, seed, block, recip, claim_list, &d_peel->norder, n, d_lover, nullptr, 0);
+          ctx->launches++;
+          S615_CU(cudaMemcpyAsync(&h.norder, &d_peel->norder, 8, cudaMemcpyDeviceToHost, st));
+          S615_CU(cudaStreamSynchronize(st));
+          const u64 L = h.norder - total;
+          const double claim_ms = trace.on ? ms_since(t_claim) : 0.0;
+          const auto t_apply = TClock::now();
+          if (L == 0) break;
+          unsigned long long h_next = 0;
+          u32 h_lover = 0;
+          S615_CU(cudaMemsetAsync(d_nnext, 0, 8, st));
+          S615_CU(cudaMemsetAsync(d_lover, 0, 4, st));
+          k_apply_list<<<blocks_for(L, 256 * kApplyPer), 256, 0, st>>>(
+              claim_list.at(total), L, W, K, seed, block, recip, fr[cur ^ 1], d_nnext, fcap, d_lover,
+              nullptr, 0);
+          ctx->launches++;
+          S615_CU(cudaGetLastError());
+          S615_CU(cudaMemcpyAsync(&h_next, d_nnext, 8, cudaMemcpyDeviceToHost, st));
+          S615_CU(cudaMemcpyAsync(&h_lover, d_lover, 4, cudaMemcpyDeviceToHost, st));
+          S615_CU(cudaStreamSynchronize(st));
+          if (trace.on) rounds_trace.push_back({(double)ncand, (double)L, claim_ms, ms_since(t_apply)});
+          total += L;
+          off.push_back(total);
+          cur ^= 1;
+          ncand = h_next;
+          over = h_lover != 0;
+        }
+        if (over) {   // candidates overflowed: the next round scans every cell
           cand = CellList{nullptr, nullptr};
           ncand = m;
           S615_CU(cudaMemsetAsync(d_lover, 0, 4, st));
@@ -1219,7 +1288,6 @@ int build_xor_device(s615_ctx* ctx, const u64* d_pair_vals, u64 n_vals, const u6
           }
         } else {
           cand = fr[cur];
-          ncand = h_n[1];
           if (ncand == 0) break;   // nothing became count 1: the peel is over
         }
       }
