@@ -416,7 +416,7 @@ int s615_check_flags(s615_ctx* ctx, uint32_t* flags) {
   if (!ctx || !flags) return S615_E_ARG;
   cudaSetDevice(ctx->device);
   S615_CU(cudaDeviceSynchronize());   // the kernels that may have set a flag are done
-  *flags = check_take_peel() | check_take_peel617() | check_take_table() | check_take_xor_build();
+  *flags = check_take_peel() | check_take_peel617() | check_take_staged() | check_take_table() | check_take_xor_build();
   return S615_OK;
 }
 

@@ -310,6 +310,7 @@ void pool_release(s615_ctx* ctx);
 // build), one per compiled file whose kernels check their indices.
 unsigned check_take_peel();
 unsigned check_take_peel617();
+unsigned check_take_staged();
 unsigned check_take_table();
 unsigned check_take_xor_build();
 // Grow-only scratch slot k of the context (no free, so no device-wide sync

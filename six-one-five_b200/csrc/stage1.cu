@@ -221,6 +221,7 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
   b->cap_items = b->items_bytes / sizeof(u64);
   b->n_items = n_items;
   b->n_main = n_items;
+  b->h2d_bytes = n_units * sizeof(DevUnit) + n_items * sizeof(u64);   // s615_batch_size: the records' size
   if (n_units) {
     S615_CU(cudaMemcpyAsync(d_io, io.data(), n_units * 4, cudaMemcpyHostToDevice, st));
     k_s1_items<<<(u32)((n_units + 255) / 256), 256, 0, st>>>(b->d_units, (u32)n_units, d_io, b->d_items);

@@ -161,7 +161,9 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   }
   const bool staged = lb < 0;
   if (staged) {   // 4 bits for the staged probe, when its slices (staged.cuh) fit L2
-    if (t.bytes < ((size_t)1 << 30) || t.hdr.r < 4 || m / 2 / 3 / 16 > kStageSlice) return S615_OK;
+    // Below 16 bits the filter's own false positives (2^-r of the keys) fill the
+    // chunk's Bloom filter, and the last pass would probe most keys again.
+    if (t.bytes < ((size_t)1 << 30) || t.hdr.r < 16 || m / 2 / 3 / 16 > kStageSlice) return S615_OK;
     lb = 2;
   }
   const u32 per = 32u >> lb;
