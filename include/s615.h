@@ -338,11 +338,15 @@ int s615_unit_status(const s615_unit* unit);
  * (the filter's false positives at rejected points are not probed) and
  * calls/gated/probes count the sharper gate.  Ignored with S615_F_NO_GATE. */
 #define S615_F_SHARP 8u
-/* Launch the peel kernels without their L2-persisting access window (no
- * counterpart in the reference).  By default a table whose cells fit the
- * device's persisting L2 set-aside is marked persisting for the launch, and a
- * larger table's launches mark the gate pattern block instead; results are
- * the same either way.  This flag exists to measure the window. */
+/* Accepted, and without effect: no launch carries an L2-persisting access
+ * window (no counterpart in the reference).  A window needs a set-aside, which
+ * is taken from every other access of the process from then on, 16 MB at
+ * least; the launches used to ask for the device's limit, 79 MB of the 126.
+ * A table that fits the set-aside stays in L2 by itself (config 1's, 1.9 MB:
+ * 26.55 us a pass with the window, 26.37 without; N = 1,500 to 3,900 the same
+ * within 3%), while what streams through L2 lost a fifth to a half: the staged
+ * probe of the 3.2M band 247 -> 208 ms without the set-aside, the builder's
+ * phases at N = 48,000 564 -> 405 ms. */
 #define S615_F_NO_L2_WINDOW 16u
 
 /* The peel of a mixed batch of units (classes 2-5 and 7) in one persistent

@@ -558,15 +558,8 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
     ++P.sub_log2;
   const size_t need = ((n_here << P.sub_log2) + kWarps - 1) / kWarps;
   if ((size_t)grid > need) grid = (int)need;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemTotal;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  cfg.attrs = attr;
-  cfg.numAttrs = (unsigned)l2_window(ctx, tv, flags, attr);
-  S615_CU(cudaLaunchKernelEx(&cfg, k_peel<kSharp, kSet, kMode>, P));
+  // (no L2 access-policy window: see s615.h, S615_F_NO_L2_WINDOW)
+  k_peel<kSharp, kSet, kMode><<<grid, kThreads, kSmemTotal, st>>>(P);
   ctx->launches++;
   S615_CU(cudaGetLastError());
   return S615_OK;
