@@ -180,13 +180,14 @@ void free_table(s615_ctx* ctx, DevTable& t) {
   t.d_cells = nullptr;
   t.bytes = 0;
   dev_free(ctx, t.d_plane, t.plane_bytes);
-  t.d_plane = nullptr;
-  t.plane_bytes = 0;
+  dev_free(ctx, t.d_splane, t.splane_bytes);
+  t.d_plane = t.d_splane = nullptr;
+  t.plane_bytes = t.splane_bytes = 0;
 }
 
 // Device bytes of a table or of every shard of a set.
 size_t table_bytes(const DevTable& t) {
-  size_t b = t.bytes + t.plane_bytes;
+  size_t b = t.bytes + t.plane_bytes + t.splane_bytes;
   for (const DevTable& p : t.parts) b += p.bytes;
   return b;
 }

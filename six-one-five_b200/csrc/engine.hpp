@@ -97,13 +97,13 @@ struct DevTable {
   u32 shard_lo = 0;              // parts[i] is shard shard_lo + i of hdr.shard_count
   void* d_views = nullptr;       // one TableView per shard of the set in HBM (owned ones set)
   u32 groups = 0;                // probe passes over a set (0: from its size)
-  // The plane: the low 2^plane_lb bits of every cell, packed into 32-bit words
-  // (a single table whose plane fits L2 far better than its cells, or, with
-  // plane_staged, one that the staged probe reads slice by slice; table.cu).
-  void* d_plane = nullptr;
-  size_t plane_bytes = 0;
+  // Planes: the low bits of every cell, packed into 32-bit words (a single table
+  // only; table.cu).  d_plane holds 2^plane_lb bits and is probed before the cells:
+  // it fits L2 far better.  d_splane holds 4 and is what the staged probe reads,
+  // slice by slice.
+  void *d_plane = nullptr, *d_splane = nullptr;
+  size_t plane_bytes = 0, splane_bytes = 0;
   u32 plane_lb = 0;
-  bool plane_staged = false;
 };
 
 // The staged probe (staged.cu) reads a plane in slices; the largest may have

@@ -313,7 +313,12 @@ u64 stage_warps(const s615_ctx* ctx) { return (u64)ctx->num_sms * 64; }
 // six launches are small beside it, few enough that most chunks of a search hold
 // no key of the table (about one in 1e9) and skip the resolve pass.
 constexpr u64 kMaxChunkKeys = 1ull << 28, kMinChunkKeys = 1ull << 26;
-constexpr double kMinKeys = 1e8;
+// The least keys for which the stages pay: below, six launches and part-filled
+// pages cost more than the scattered reads.  Direct / staged, ms, class-5 units:
+// 1e7 keys 0.74 / 0.69 (N = 42,000), 0.55 / 0.60 (31,000); 2e7 1.47 / 1.07 and
+// 0.99 / 0.91; 2.4e7 1.72 / 1.44 (76,667), but 1.64 / 1.74 with a key of the table
+// among them, when the resolve pass runs; 4.4e7 2.93 / 2.22; 1e8 7.2 / 4.4.
+constexpr double kMinKeys = 2.5e7;
 
 // Two spaces in turn: the emitted pages, stage 1's runs, stage 2's in the
 // pages' place.

@@ -126,13 +126,31 @@ TableView view_of(const DevTable& t) {
   v.r = t.hdr.r;
   v.layout = (u32)t.layout;
   v.cell_bytes = (u32)t.cell_bytes;
-  v.plane = t.plane_staged ? nullptr : static_cast<const u32*>(t.d_plane);
-  v.splane = t.plane_staged ? static_cast<const u32*>(t.d_plane) : nullptr;
+  v.plane = static_cast<const u32*>(t.d_plane);
+  v.splane = static_cast<const u32*>(t.d_splane);
   v.plane_bytes = t.plane_bytes;
   v.plane_lb = t.plane_lb;
   v.plane_mask = (u32)((1ull << (1u << t.plane_lb)) - 1);
   if (t.hdr.n_keys == 0 || t.hdr.m_cells < 3) v.block = 0;
   return v;
+}
+
+// The low 2^lb bits of t's cells; *p stays null when there is no room.
+static int make_plane(s615_ctx* ctx, const DevTable& t, int lb, cudaStream_t st, void** p, size_t* bytes) {
+  const u64 m = t.hdr.m_cells, per = 32u >> lb, words = (m + per - 1) / per;
+  if (dev_alloc_once(ctx, p, words * sizeof(u32))) return S615_OK;
+  k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
+                                                     t.hdr.r, m, (u32)lb, static_cast<u32*>(*p), words);
+  ctx->launches++;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    dev_free(ctx, *p, words * sizeof(u32));
+    *p = nullptr;
+    return cuda_status(e);
+  }
+  *bytes = words * sizeof(u32);
+  return S615_OK;
 }
 
 // A probe costs three scattered reads of cells, or with a plane of b bits
@@ -142,10 +160,15 @@ TableView view_of(const DevTable& t) {
 // bit) the plane is mostly read from DRAM itself: a 4-bit plane of 468 MB gave
 // a class-5 pass 7% and took 14% from a mixed one.  Measured, ps per probe
 // through the cells alone / with the plane: class 5, N = 12,000 (4 bits) 65.5
-// / 43.6, 20,000 (2 bits) 63.2 / 34.4, 24,000 (2 bits) 63.2 / 38.1, 31,000 (1
-// bit) 63.1 / 46.5, 37,000 (1 bit) 63.2 / 54.4; (6,1,7), N = 10,476 (8 bits) 54.7 /
-// 14.6.  Three reads of a 64 MB plane are 10.5 ps.
+// / 43.6, 20,000 (2 bits) 63.2 / 25.5, 24,000 (2 bits) 63.2 / 30.2, 31,000 (1
+// bit) 63.1 / 42.9, 36,000 (1 bit) 63.2 / 47.5; (6,1,7), N = 10,476 (8 bits) 54.7 /
+// 14.  Three reads of a 64 MB plane are 10.5 ps.
 constexpr double kPlaneMaxMB = 112;
+// The staged probe takes 34 to 37 ps a key, whatever the table (N = 20,000 to
+// 76,667, 2e8 keys), so tables whose probe costs more by this count get its plane
+// as well, for their large batches: N = 28,000 (1 bit) 42.6 -> 34.3 ps, 36,000 48.0
+// -> 36.0, 48,000 63.1 -> 35.8; N = 24,000 (2 bits, 30.7 ps) would lose.
+constexpr double kStagedPs = 38;
 int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   const u64 m = t.hdr.m_cells;
   if (!t.d_cells || t.hdr.n_keys == 0 || m < 3) return S615_OK;
@@ -159,35 +182,19 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
     const double ps = 3 * read_ps(mb) + cell_ps / (double)(1u << bits);
     if (mb <= kPlaneMaxMB && ps < best) { best = ps; lb = k; }
   }
-  const bool staged = lb < 0;
-  if (staged) {   // 4 bits for the staged probe, when its slices (staged.cuh) fit L2
-    // Below 16 bits the filter's own false positives (2^-r of the keys) fill the
-    // chunk's Bloom filter, and the last pass would probe most keys again.
-    if (t.bytes < ((size_t)1 << 30) || t.hdr.r < 16 || m / 2 / 3 / 16 > kStageSlice) return S615_OK;
-    lb = 2;
+  if (lb >= 0) {
+    if (const int s = make_plane(ctx, t, lb, st, &t.d_plane, &t.plane_bytes)) return s;
+    t.plane_lb = (u32)lb;
   }
-  const u32 per = 32u >> lb;
-  const u64 words = (m + per - 1) / per;
-  void* p = nullptr;
+  // The staged probe's plane, when its slices (staged.cuh) fit L2.  Below 16 bits
+  // the filter's own false positives (2^-r of the keys) fill the chunk's Bloom
+  // filter, and the last pass would probe most keys again.
+  if ((t.d_plane ? best : cell_ps) < kStagedPs || t.hdr.r < 16 || m / 2 / 3 / 16 > kStageSlice)
+    return S615_OK;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
-  // no room, or room that a search will want: the cells alone
-  if (staged && 4 * words * sizeof(u32) > free_b) return S615_OK;
-  if (dev_alloc_once(ctx, &p, words * sizeof(u32))) return S615_OK;
-  k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
-                                                     t.hdr.r, m, (u32)lb, static_cast<u32*>(p), words);
-  ctx->launches++;
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    dev_free(ctx, p, words * sizeof(u32));
-    return cuda_status(e);
-  }
-  t.d_plane = p;
-  t.plane_bytes = words * sizeof(u32);
-  t.plane_lb = (u32)lb;
-  t.plane_staged = staged;
-  return S615_OK;
+  if (4 * (m / 2) > free_b) return S615_OK;   // room that a search will want
+  return make_plane(ctx, t, 2, st, &t.d_splane, &t.splane_bytes);
 }
 
 int launch_xor_query(s615_ctx* ctx, const TableView& tv, const u64* d_keys, size_t n,
