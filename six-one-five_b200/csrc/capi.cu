@@ -958,7 +958,7 @@ static int fill_on_device(s615_ctx* ctx, const s615_unit* units, size_t n, s615_
   std::vector<char> other(nt, 0);
   run_threads(nt, [&](size_t t) {
     for (size_t i = n * t / nt, hi = n * (t + 1) / nt; i < hi; ++i) {
-      if (units[i].cls < 2 || units[i].cls > 5) { other[t] = 1; return; }
+      if ((units[i].cls < 1 || units[i].cls > 5) && units[i].cls != S615_CLS_617_FIND4) { other[t] = 1; return; }
       stage[i] = units[i];
     }
   });
@@ -966,8 +966,8 @@ static int fill_on_device(s615_ctx* ctx, const s615_unit* units, size_t n, s615_
     if (o) return S615_OK;
   if (!ctx->aux) S615_CU(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
   const u32 job_rows = job_rows_for(ctx, n);
-  void *raw = nullptr, *tot = nullptr;
-  size_t raw_bytes = 0, tot_bytes = 0;
+  void *raw = nullptr, *tot = nullptr, *second = nullptr, *scratch = nullptr;
+  size_t raw_bytes = 0, tot_bytes = 0, second_bytes = 0, scratch_bytes = 0;
   FillTotals h{};
   int s = batch_buffers(ctx, b, n, 0);
   if (!s) s = pool_get(ctx, n * sizeof(s615_unit), &raw, &raw_bytes);
@@ -991,18 +991,27 @@ static int fill_on_device(s615_ctx* ctx, const s615_unit* units, size_t n, s615_
     b->item_rows = kItemRows >> q;
     b->parts3 = !set && q == 2 ? 4u : 1u;
     b->n_units = n;
-    b->n_items = b->n_main = h.items5[q] + h.items234[q] * b->parts3 + h.jobs;
+    b->n_main = h.items5[q] + h.items234[q] * b->parts3 + h.jobs;
+    b->n_items = b->n_main + h.find4;
     b->est_keys = h.keys;
     b->host_items_valid = false;
     b->h2d_bytes = n * sizeof(s615_unit);
     s = batch_buffers(ctx, b, n, b->n_items);
+    if (!s && h.find4) s = pool_get(ctx, h.find4 * sizeof(u64), &second, &second_bytes);
+    if (!s && h.find4) s = pool_get(ctx, order_items_scratch(ctx, h.find4), &scratch, &scratch_bytes);
+    auto* d_second = static_cast<u64*>(second);
     if (!s && b->n_items)
       s = launch_items(ctx, d_raw, b->d_units, (u32)n, job_rows, b->item_rows, b->parts3, b->d_items,
-                       b->n_items, d_tot, ctx->aux);
+                       b->n_main, d_second, h.find4, d_tot, ctx->aux);
+    // heaviest first, as below
+    if (!s && h.find4)
+      s = order_items(ctx, d_second, b->d_items + b->n_main, h.find4, scratch, ctx->aux);
   }
   if (cudaStreamSynchronize(ctx->aux) != cudaSuccess && !s) s = S615_E_DEVICE;
   pool_put(ctx, raw, raw_bytes);
   pool_put(ctx, tot, tot_bytes);
+  pool_put(ctx, second, second_bytes);
+  pool_put(ctx, scratch, scratch_bytes);
   if (s == S615_E_OOM) return S615_OK;   // the host's way needs less
   *done = true;
   return s;

@@ -358,17 +358,19 @@ S615_HD double unit_keys(const DevUnit& d) {
   return rows * (d.cls == 5 ? 0.0243 * d.nres2 * d.fmax2 / 64 : 0.0043 * d.lim);
 }
 
-// Unit records and work items of classes 2-5 made on the device (pack.cu).
+// Unit records and work items of classes 1-5 and 8 made on the device (pack.cu).
 struct FillTotals {
   unsigned long long items5[3], items234[3];   // row chunks of 64, 32, 16 rows
   unsigned long long jobs, placed;             // job items; items written
+  unsigned long long find4, placed4;           // the same of the second kernel's items
   double keys;
   u32 bad, pad;                                // a unit was refused
 };
 int launch_pack(s615_ctx* ctx, const s615_unit* d_raw, u32 n, u32 job_rows, DevUnit* units,
                 FillTotals* tot, cudaStream_t st);
 int launch_items(s615_ctx* ctx, const s615_unit* d_raw, const DevUnit* units, u32 n, u32 job_rows,
-                 u32 rows, u32 parts3, u64* items, u64 n_items, FillTotals* tot, cudaStream_t st);
+                 u32 rows, u32 parts3, u64* items, u64 n_items, u64* second, u64 n_second,
+                 FillTotals* tot, cudaStream_t st);
 
 // Device verifier; see verify.cu.
 int verify_device(s615_ctx* ctx, const s615_unit* units, size_t n_units, const s615_hit* hits,

@@ -1,17 +1,19 @@
 // pack.cu -- unit records and work items made on the device.
 //
 // make_dev_unit (host_math.cpp) and unit_items (engine.hpp) for the units of
-// classes 2-5, of all three kinds, one thread per unit: the caller's 72-byte
-// records cross the bus instead of 224-byte ones and 8-byte items, and the host
-// works out no residues.  (214,000 reduced-T jobs: 8 of the 10 ms of a call were
-// the host's packing and a 48 MB upload.)  Batches with units of other classes
-// are packed on the host.
+// classes 1-5, of all three kinds, and (6,1,7) find4 jobs, one thread per unit: the
+// caller's 72-byte records cross the bus instead of 224-byte ones and 8-byte
+// items, and the host works out no residues.  (214,000 reduced-T jobs: 8 of the
+// 10 ms of a call were the host's packing and a 48 MB upload, 11 -> 4.4 ms with
+// class-1 jobs among them; 100,001 (6,1,7) find4 jobs 25.2 -> 21.5 ms.)  Batches with
+// (6,1,7) class-5 candidates are packed on the host.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
 
 #include "pack.cuh"
+#include "s615_device.cuh"
 
 namespace s615 {
 
@@ -66,18 +68,84 @@ __device__ __forceinline__ bool job_row(const s615_unit& u, bool* find2) {
   return u.cls == 5 || ((u.base[0] | u.base[1]) != 0 && (u.base[1] >> 57) == 0);   // 0 < T < 2^121
 }
 
-// make_dev_unit for classes 2-5: S615_OK (with *skip for a dropped unit) or
+// Class 1, target T in 1 .. 2^126 - 1: the c4 window [least c with 4 c^6 >= T,
+// min(T^(1/6), lim)]; true if it is empty (4 c^6 >= T iff c^6 > floor((T - 1) / 4)).
+__device__ bool find4_window(u128 T, u32 lim, DevUnit* out) {
+  const u32 hi4 = min(iroot6_u128(T), lim), lo4 = iroot6_u128((T - 1) >> 2) + 1;
+  if (hi4 < 1 || lo4 > hi4) return true;
+  out->cls = 1;
+  out->lim = lim;
+  out->base_lo = (u64)T;
+  out->base_hi = (u64)(T >> 64);
+  out->fmax1 = hi4;
+  out->fmax2 = lo4;
+  out->nres1 = 1;
+  return false;
+}
+// make_dev_unit1: a class-1 Stage-1 unit or plant.
+__device__ int pack_find4(const s615_unit& in, DevUnit* out, bool* skip) {
+  W3 R;
+  u32 lim = in.lim;
+  if (in.kind == 0) {
+    const u64 B = in.B, u = in.u;
+    if (B < 2 || B > kMaxB || u == 0) return S615_E_FORMAT;
+    if (u >= B) { *skip = true; return S615_OK; }
+    R = d_pow6(B);
+    d_sub(R, d_pow6(u));
+    lim = (u32)((B - 1) / 42);
+  } else if (in.kind == 1) {
+    R = W3{{in.base[0], in.base[1], in.base[2]}};
+    if (in.lim >= (1u << 21)) return S615_E_FORMAT;
+  } else {
+    return S615_E_FORMAT;
+  }
+  if ((R.l[0] | R.l[1] | R.l[2]) == 0) return S615_E_FORMAT;
+  u64 rem = 0;   // T = R / 42^6, exactly
+#pragma unroll
+  for (int i = 2; i >= 0; --i) {
+    const u128 d = ((u128)rem << 64) | R.l[i];
+    R.l[i] = (u64)(d / kM42);
+    rem = (u64)(d % kM42);
+  }
+  if (rem != 0 || R.l[2] != 0 || (R.l[1] >> 62) != 0) return S615_E_FORMAT;
+  out->B = in.B; out->u = in.u;
+  *skip = find4_window(((u128)R.l[1] << 64) | R.l[0], lim, out);
+  return S615_OK;
+}
+// make_dev_unit8: a (6,1,7) find4 job.
+__device__ int pack_617_find4(const s615_unit& in, DevUnit* out) {
+  if (in.kind != 0 || in.base[2] != 0 || (in.base[1] >> 62) != 0) return S615_E_FORMAT;
+  if (in.lim >= (1u << 21) || in.fmax2 < 1 || in.fmax1 < in.fmax2 || in.fmax1 > in.lim)
+    return S615_E_FORMAT;
+  out->cls = S615_CLS_617_FIND4;
+  out->B = in.B; out->u = in.u; out->w = in.w;
+  out->base_lo = in.base[0];
+  out->base_hi = in.base[1];
+  out->lim = in.lim;
+  out->fmax1 = in.fmax1;
+  out->fmax2 = in.fmax2;
+  out->nres1 = 1;
+  out->pad1 = in.res_e;
+  out->pad2 = in.res_d;
+  return S615_OK;
+}
+
+// make_dev_unit for the classes above: S615_OK (with *skip for a dropped unit) or
 // S615_E_FORMAT, in its order of checks.
 __device__ int pack_one(const Roots& R, const s615_unit& in, DevUnit* out, bool* skip) {
   *skip = false;
   const u32 cls = in.cls;
   if (in.kind == S615_KIND_JOB) {
-    if (in.base[2] != 0) return S615_E_FORMAT;
+    if (cls < 1 || cls > 5 || in.base[2] != 0) return S615_E_FORMAT;
     const u128 T = ((u128)in.base[1] << 64) | in.base[0];
     const u64 lim = in.lim ? in.lim : (in.B ? (in.B - 1) / 42 : 0);
     if (lim > (kMaxB - 1) / 42) return S615_E_FORMAT;
     out->B = in.B; out->u = in.u;
     out->lim = (u32)lim;
+    if (cls == 1) {
+      *skip = T == 0 || (T >> 122) != 0 || find4_window(T, (u32)lim, out);
+      return S615_OK;
+    }
     u128 W;
     if (cls == 5) {
       const u128 M = (u128)15561 << 64;
@@ -104,6 +172,8 @@ __device__ int pack_one(const Roots& R, const s615_unit& in, DevUnit* out, bool*
     out->base_hi = (u64)(base >> 64);
     return S615_OK;
   }
+  if (cls == 1) return pack_find4(in, out, skip);
+  if (cls == S615_CLS_617_FIND4) return pack_617_find4(in, out);
   W3 base;
   out->cls = cls;
   out->f = cls == 2 ? 14 : cls == 3 ? 21 : cls == 4 ? 7 : 0;
@@ -198,6 +268,10 @@ __device__ __forceinline__ u32 row_items(const DevUnit& d, u32 rows) {
   }
   return n;
 }
+// Items of the second kernel: chunks of a find4 unit's c4 window.
+__device__ __forceinline__ u32 find4_items(const DevUnit& d) {
+  return d.cls == 1 || d.cls == S615_CLS_617_FIND4 ? (d.fmax1 - d.fmax2) / kC4Chunk + 1 : 0u;
+}
 // Does unit k begin a job item?  Consecutive job rows of one kind share items,
 // never across a multiple of job_rows.
 __device__ __forceinline__ bool job_start(const s615_unit* raw, u32 k, u32 job_rows) {
@@ -209,7 +283,7 @@ __device__ __forceinline__ bool job_start(const s615_unit* raw, u32 k, u32 job_r
 __global__ void k_pack(Roots R, const s615_unit* __restrict__ raw, u32 n, u32 job_rows,
                        DevUnit* __restrict__ units, FillTotals* tot) {
   const u32 k = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  u32 c5[3] = {0, 0, 0}, c3[3] = {0, 0, 0}, jobs = 0;
+  u32 c5[3] = {0, 0, 0}, c3[3] = {0, 0, 0}, jobs = 0, find4 = 0;
   double keys = 0;
   bool bad = false;
   if (k < n) {
@@ -221,13 +295,14 @@ __global__ void k_pack(Roots R, const s615_unit* __restrict__ raw, u32 n, u32 jo
     if (skip) d.cls = 0;
     units[k] = d;
     if (!bad && !skip) {
-      keys = unit_keys(d);
+      find4 = find4_items(d);
       if (d.cls == kClsJobRow) {
         jobs = job_start(raw, k, job_rows);
-      } else {
+      } else if (!find4) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) (d.cls == 5 ? c5 : c3)[i] = row_items(d, kItemRows >> i);
       }
+      if (!find4) keys = unit_keys(d);
     }
   }
 #pragma unroll
@@ -238,6 +313,7 @@ __global__ void k_pack(Roots R, const s615_unit* __restrict__ raw, u32 n, u32 jo
       c3[i] += __shfl_xor_sync(0xFFFFFFFFu, c3[i], o);
     }
     jobs += __shfl_xor_sync(0xFFFFFFFFu, jobs, o);
+    find4 += __shfl_xor_sync(0xFFFFFFFFu, find4, o);
     keys += __shfl_xor_sync(0xFFFFFFFFu, keys, o);
   }
   bad = __any_sync(0xFFFFFFFFu, bad);
@@ -247,31 +323,25 @@ __global__ void k_pack(Roots R, const s615_unit* __restrict__ raw, u32 n, u32 jo
       if (c3[i]) atomicAdd(&tot->items234[i], (unsigned long long)c3[i]);
     }
     if (jobs) atomicAdd(&tot->jobs, (unsigned long long)jobs);
+    if (find4) atomicAdd(&tot->find4, (unsigned long long)find4);
     if (keys > 0) atomicAdd(&tot->keys, keys);
     if (bad) tot->bad = 1;
   }
 }
 
-// The items of 256 units, one after another; the blocks' runs come in the order
-// in which the blocks reserve them.
-__global__ void k_items(const s615_unit* __restrict__ raw, const DevUnit* __restrict__ units, u32 n,
-                        u32 job_rows, u32 rows, u32 parts3, u64* __restrict__ items, u64 cap,
-                        FillTotals* tot) {
+// The place of this thread's c items in a run of the block's, reserved at `cursor`.
+// Every thread of the block calls this.
+__device__ __forceinline__ u64 block_place(u32 c, unsigned long long* cursor) {
   __shared__ u32 s_w[8];
   __shared__ unsigned long long s_base;
-  const u32 k = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  u32 c = 0, cls = 0;
-  if (k < n) {
-    cls = units[k].cls;
-    if (cls == kClsJobRow) c = job_start(raw, k, job_rows);
-    else if (cls) c = row_items(units[k], rows) * (cls == 5 ? 1u : parts3);
-  }
+  const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u32 incl = c;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const u32 y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
     if (lane >= (u32)o) incl += y;
   }
+  __syncthreads();
   if (lane == 31) s_w[wid] = incl;
   __syncthreads();
   u32 before = 0, all = 0;
@@ -279,9 +349,31 @@ __global__ void k_items(const s615_unit* __restrict__ raw, const DevUnit* __rest
     if (w < wid) before += s_w[w];
     all += s_w[w];
   }
-  if (threadIdx.x == 0) s_base = all ? atomicAdd(&tot->placed, (unsigned long long)all) : 0ull;
+  if (threadIdx.x == 0) s_base = all ? atomicAdd(cursor, (unsigned long long)all) : 0ull;
   __syncthreads();
-  u64 at = s_base + before + incl - c;
+  return s_base + before + incl - c;
+}
+
+// The items of 256 units, one after another; the blocks' runs come in the order
+// in which the blocks reserve them.  Find4 units' items go to `second` (to be
+// ordered by order_items), the others' to `items`.
+__global__ void k_items(const s615_unit* __restrict__ raw, const DevUnit* __restrict__ units, u32 n,
+                        u32 job_rows, u32 rows, u32 parts3, u64* __restrict__ items, u64 cap,
+                        u64* __restrict__ second, u64 cap2, FillTotals* tot) {
+  const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
+  u32 c = 0, c2 = 0, cls = 0;
+  if (k < n) {
+    cls = units[k].cls;
+    c2 = cls ? find4_items(units[k]) : 0u;
+    if (cls == kClsJobRow) c = job_start(raw, k, job_rows);
+    else if (cls && !c2) c = row_items(units[k], rows) * (cls == 5 ? 1u : parts3);
+  }
+  if (second) {   // the same for every thread
+    const u64 at2 = block_place(c2, &tot->placed4);
+    if (at2 + c2 <= cap2)
+      for (u32 i = 0; i < c2; ++i) second[at2 + i] = make_item(k, 0, i);
+  }
+  u64 at = block_place(c, &tot->placed);
   if (c == 0 || at + c > cap) return;   // cap is the total: never past it
   if (cls == kClsJobRow) {
     bool kind, other;
@@ -315,8 +407,10 @@ int launch_pack(s615_ctx* ctx, const s615_unit* d_raw, u32 n, u32 job_rows, DevU
 }
 
 int launch_items(s615_ctx* ctx, const s615_unit* d_raw, const DevUnit* units, u32 n, u32 job_rows,
-                 u32 rows, u32 parts3, u64* items, u64 n_items, FillTotals* tot, cudaStream_t st) {
-  k_items<<<(n + 255) / 256, 256, 0, st>>>(d_raw, units, n, job_rows, rows, parts3, items, n_items, tot);
+                 u32 rows, u32 parts3, u64* items, u64 n_items, u64* second, u64 n_second,
+                 FillTotals* tot, cudaStream_t st) {
+  k_items<<<(n + 255) / 256, 256, 0, st>>>(d_raw, units, n, job_rows, rows, parts3, items, n_items,
+                                           second, n_second, tot);
   ctx->launches++;
   S615_CU(cudaGetLastError());
   return S615_OK;

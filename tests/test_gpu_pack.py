@@ -1,5 +1,5 @@
 """Unit records and work items made on the device give what the host's give: the
-same units run alone (packed on the device) and with a class-1 unit beside them,
+same units run alone (packed on the device) and with a class-7 unit beside them,
 which sends the whole batch the host's way (GPU)."""
 import ctypes as C
 
@@ -33,8 +33,9 @@ def both_ways(table, units, flags=0):
     arr = (s615.Unit * (n + 1))(*units)
     lib = s615.lib()
     got_bytes, status = {}, {}
-    # a class-1 target whose window is empty: dropped, and nothing of it is counted
-    empty = s615.make_plant1((1, 1, 1, 1), lim=0)
+    # a (6,1,7) candidate with u >= B: dropped, and nothing of it is counted
+    empty = s615.Unit()
+    empty.cls, empty.B, empty.u, empty.w = 7, 5, 5 + 9 * 729, 5 + 117649
     assert lib.s615_unit_status(C.byref(empty)) == 1
     arr[n] = empty
     out = []
@@ -104,10 +105,42 @@ def test_jobs_with_gaps(table):
         both_ways(table, out[:cut])
 
 
+def test_find4_units(table):
+    """Class 1 as Stage-1 units, jobs and plants, and (6,1,7) find4 jobs: alone, among the
+    others, with empty windows and targets at the ends of what is taken."""
+    units = units_of(*s615.jobs617_band([71001, 71003], (1, 2, 3, 4)))[:1500]
+    stage1 = []
+    for c, B, u in W.mixed_units(120, 5, 40000, 84000, mix={1: 0.7, 4: 0.3}):
+        x = s615.Unit()
+        x.cls, x.B, x.u = c, B, u
+        stage1.append(x)
+    jobs, nj, _ = s615.expand_units(W.mixed_units(30, 6, 60000, 84000, mix={1: 0.5, 4: 0.5}))
+    plants = [s615.make_plant1((a, 700, 900, 1900), lim=1999) for a in (1, 500, 699)]
+    plants.append(s615.make_plant1((1, 1, 1, 1), lim=0))
+    plants.append(s615.make_plant1((1, 1, 1, 1), lim=1))
+    edge = []
+    for T in (1, 4, 5, 64, 4 * 7**6, 4 * 7**6 + 1, 2**122 - 1, 2**122, 0):
+        j = s615.Unit()
+        j.cls, j.kind, j.lim, j.B, j.u = 1, 2, 1999, 83999, 5
+        j.base[0], j.base[1] = T & (2**64 - 1), T >> 64
+        edge.append(j)
+    # lim = 1999 leaves the last targets' windows empty; the hits are those of few probes
+    mixed = edge + plants + stage1 + units_of(jobs, min(nj, 900)) + units
+    assert {x.cls for x in mixed} >= {1, 4, 8}
+    hits, ctr = both_ways(table, mixed)
+    assert ctr[2] > 0
+    both_ways(table, units)
+    both_ways(table, edge * 20)
+
+
 def test_a_refused_unit_refuses_the_batch(table):
     eng, tid = table
     good = units_of(*W.unit_array(W.cls5_units(20000, 24000)[:200], [], N))
     for bad in (dict(cls=5, B=20005, u=8), dict(cls=2, B=40000001, u=5), dict(cls=4, B=1, u=5),
+                dict(cls=1, B=20001, u=5), dict(cls=1, kind=1, B=20001, u=5, base0=12345),
+                dict(cls=1, kind=1, B=20001, u=5, lim=1 << 21, base0=5489031744),
+                dict(cls=8, kind=1, B=20001, u=5), dict(cls=8, B=20001, u=5, fmax1=3, fmax2=4, lim=9),
+                dict(cls=8, kind=2, B=20001, u=5),
                 dict(cls=3, kind=3, B=20001, u=5), dict(cls=5, kind=2, B=20001, u=5, base2=1),
                 dict(cls=5, kind=1, B=20001, u=5, base0=12345)):
         x = s615.Unit()
