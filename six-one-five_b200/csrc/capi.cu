@@ -181,13 +181,14 @@ void free_table(s615_ctx* ctx, DevTable& t) {
   t.bytes = 0;
   dev_free(ctx, t.d_plane, t.plane_bytes);
   dev_free(ctx, t.d_splane, t.splane_bytes);
-  t.d_plane = t.d_splane = nullptr;
-  t.plane_bytes = t.splane_bytes = 0;
+  if (t.eplane_bytes) dev_free(ctx, t.d_eplane, t.eplane_bytes);
+  t.d_plane = t.d_splane = t.d_eplane = nullptr;
+  t.plane_bytes = t.splane_bytes = t.eplane_bytes = 0;
 }
 
 // Device bytes of a table or of every shard of a set.
 size_t table_bytes(const DevTable& t) {
-  size_t b = t.bytes + t.plane_bytes + t.splane_bytes;
+  size_t b = t.bytes + t.plane_bytes + t.splane_bytes + t.eplane_bytes;
   for (const DevTable& p : t.parts) b += p.bytes;
   return b;
 }

@@ -99,15 +99,16 @@ struct DevTable {
   u32 groups = 0;                // probe passes over a set (0: from its size)
   // Planes: the low bits of every cell, packed into 32-bit words (a single table
   // only; table.cu).  d_plane holds 2^plane_lb bits and is probed before the cells:
-  // it fits L2 far better.  d_splane holds 4 and is what the staged probe reads,
-  // slice by slice.
-  void *d_plane = nullptr, *d_splane = nullptr;
-  size_t plane_bytes = 0, splane_bytes = 0;
+  // it fits L2 far better.  d_splane is what the staged probe reads, slice by slice:
+  // 4 bits, above the lowest if there is d_eplane (perhaps d_plane itself), which
+  // holds that one: the staged probe's keys go through it first.
+  void *d_plane = nullptr, *d_splane = nullptr, *d_eplane = nullptr;
+  size_t plane_bytes = 0, splane_bytes = 0, eplane_bytes = 0;   // eplane_bytes 0: d_plane's
   u32 plane_lb = 0;
 };
 
 // The staged probe (staged.cu) reads a plane in slices; the largest may have
-// this many bytes and, with the pages that stream past, stay in L2 (scattered
+// this many bytes and, with the keys that stream past, stay in L2 (scattered
 // reads keep their full rate up to a 64 MB footprint, 0.8 of it at 80 MB).
 constexpr u64 kStageSlice = 80ull << 20;
 
@@ -133,7 +134,7 @@ struct TableView {
   u32 groups, pad;      // passes over the set
   u64 bytes;            // bytes of cells (a single table; 0 for a set)
   const u32* plane;     // low 2^plane_lb bits of each cell (null: none)
-  const u32* splane;    // the same, for the staged probe only
+  const u32 *splane, *eplane;   // the staged probe's
   u64 plane_bytes;
   u32 plane_lb, plane_mask;   // plane_mask = 2^(2^plane_lb) - 1
 };
@@ -207,7 +208,7 @@ struct s615_batch {
 };
 
 namespace s615 {
-// The staged probe's pages and chunk counters: one space per context, handed
+// The staged probe's key lists and chunk counters: one space per context, handed
 // from run to run (on any stream) through the event; given back with
 // s615_run's kept batch.
 struct StageSpace {

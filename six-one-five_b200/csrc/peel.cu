@@ -83,17 +83,20 @@ struct PeelParams {
   u32 parts3_log2;         // log2 of the items per class 2-4 row chunk (1 or 4 items)
   u32 item_lo;             // first item of this launch (its items: [item_lo, n_items))
   u32 sub_log2;            // each item goes out as 2^sub_log2 parts of its rows
-  u32 sb;                  // kEmit: a bucket is 2^sb cells
-  StagePages pages;        // kEmit: where keys go
+  StageRuns list;          // kEmit: where keys go
   StageChunk* chunk;       // kEmit, kResolve
 };
 
 // What a full batch of gate survivors meets.
 enum : int {
   kProbe = 0,     // the xor probe, hits recorded
-  kEmit = 1,      // the staged probe's first step: keys to pages by first cell
+  kEmit = 1,      // the staged probe's first step: keys to lists
+  kEmitPlane = 3, // kEmit, for the keys that a plane leaves
   kResolve = 2,   // its last: the probe again, for the keys in the chunk's Bloom filter
 };
+
+template <int kMode>
+constexpr bool kEmits = kMode == kEmit || kMode == kEmitPlane;
 
 // cls5 pattern words (sharp or not) then the find3 ones, then the warp slices
 // (which start on a 16-byte boundary: the row records are 16-byte aligned).
@@ -103,7 +106,7 @@ constexpr size_t smem_pat() {
 }
 template <bool kSharp, int kMode>
 constexpr size_t smem_total() {
-  return smem_pat<kSharp>() + kWarps * (sizeof(WarpT<kSharp>) + (kMode == kEmit ? sizeof(WarpHold) : 0));
+  return smem_pat<kSharp>() + kWarps * (sizeof(WarpT<kSharp>) + (kEmits<kMode> ? sizeof(WarpHold) : 0));
 }
 static_assert(sizeof(WarpSmem) % 8 == 0, "the held keys follow the warp slices");
 
@@ -122,24 +125,28 @@ struct ItemCtx {
   u32 cls, unit_id, r0, mod, j0, f;   // job items: unit_id = index of the first unit
 };
 
-// kEmit: a key whose bucket has no page left is probed where it is.
+// kEmit: a key that its list has no room for is probed where it is.
 struct DirectProbe {
   const TableView& tv;
   StageChunk* chunk;
-  __device__ __forceinline__ void operator()(u32, u64 h) const {
+  __device__ __forceinline__ void operator()(u64 h) const {
     if (contains_hash<false>(tv, h)) stage_positive(chunk, h);
   }
 };
 
+// kEmit: a warp's list (neighbouring warps take different ones).
+__device__ __forceinline__ u32 stage_list() {
+  return (blockIdx.x * kWarps + (threadIdx.x >> 5)) % kStageLists;
+}
+
 // Probe the ring entries [head, head+cnt) (one per lane).
 template <bool kSet, int kMode>
 __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem& W, u32 head,
-                                            u32 cnt, const ItemCtx& I, u32 lane, StageOpen& S,
+                                            u32 cnt, const ItemCtx& I, u32 lane, u32& held,
                                             WarpHold* H) {
-  if constexpr (kMode == kEmit) {
-    const bool act = lane < cnt;
+  if constexpr (kEmits<kMode>) {
+    bool act = lane < cnt;
     u64 h = 0;
-    u32 b = 0;
     if (act) {
       const u32 ent = W.ring[(head + lane) & (kQ - 1)];
       const u32 k = ent & 0x3FFFFu, r = (ent >> 18) & 63u, di = ent >> 24;
@@ -148,9 +155,15 @@ __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem&
       if (I.cls == 5) key = (u64)(((((u128)R.whi << 64) | R.wlo) - pow6_small((u64)W.d0s[di] + 64ull * k)) >> 6);
       else key = R.wlo - (u64)pow6_small((u64)R.a + k);
       h = mix64(key + P.tv.seed);
-      b = (u32)(fast_mod(h, P.tv.block, P.tv.recip) >> P.sb);
+      if constexpr (kMode == kEmitPlane) {   // the keys that the table's own plane leaves
+        u64 c[3];
+        cell_indices(h, P.tv.block, P.tv.recip, c);
+        act = S615_CHECK(c[0] < 3 * P.tv.block && c[1] < 3 * P.tv.block && c[2] < 3 * P.tv.block, kChkCell) &&
+              !((load_plane(P.tv, c[0]) ^ load_plane(P.tv, c[1]) ^ load_plane(P.tv, c[2]) ^ (u32)h) &
+                P.tv.plane_mask);
+      }
     }
-    stage_push(P.pages, *H, S, act, b, h, lane, DirectProbe{P.tv, P.chunk});
+    stage_push(P.list, stage_list(), *H, held, act, h, lane, DirectProbe{P.tv, P.chunk});
     return;
   }
   if (lane >= cnt) return;
@@ -195,7 +208,7 @@ __device__ __forceinline__ void probe_batch(const PeelParams& P, const WarpSmem&
 template <bool kSet, int kMode>
 __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 m, u32 di, u32 r,
                                           u32 kbase, u32& head, u32& qlen, const ItemCtx& I,
-                                          u32 lane, StageOpen& S, WarpHold* H) {
+                                          u32 lane, u32& held, WarpHold* H) {
   while (__any_sync(0xFFFFFFFFu, m != 0)) {
     const bool has = m != 0;
     const u32 bit = has ? (u32)(__ffs(m) - 1) : 0u;
@@ -205,7 +218,7 @@ __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 
     qlen += __popc(ballot);
     if (qlen >= 32u) {
       __syncwarp();
-      probe_batch<kSet, kMode>(P, W, head, 32u, I, lane, S, H);
+      probe_batch<kSet, kMode>(P, W, head, 32u, I, lane, held, H);
       __syncwarp();
       head = (head + 32u) & (kQ - 1);
       qlen -= 32u;
@@ -214,7 +227,7 @@ __device__ __forceinline__ void push_bits(const PeelParams& P, WarpSmem& W, u32 
 }
 
 template <bool kSharp, bool kSet, int kMode = kProbe>
-__global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5) k_peel(PeelParams P) {
+__global__ void __launch_bounds__(kThreads, kSharp ? 3 : kEmits<kMode> ? 4 : 5) k_peel(PeelParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
   if constexpr (kMode == kResolve) {
     if (P.chunk->positives == 0) return;   // nothing in this chunk: the usual case
@@ -230,9 +243,9 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5)
 
   const u128 inv21 = ((u128)P.inv21_hi << 64) | P.inv21_lo;
   u64 my_calls = 0, my_pos = 0, my_probes = 0;
-  StageOpen S;
+  u32 held = 0;
   WarpHold* H = nullptr;
-  if constexpr (kMode == kEmit)
+  if constexpr (kEmits<kMode>)
     H = reinterpret_cast<WarpHold*>(smem + smem_pat<kSharp>() + kWarps * sizeof(WarpT<kSharp>)) + warp;
 
   for (;;) {
@@ -376,12 +389,12 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5)
                 m &= lowmask;
               }
               my_probes += __popc(m);
-              push_bits<kSet, kMode>(P, W, m, di, r, kbase, head, qlen, I, lane, S, H);
+              push_bits<kSet, kMode>(P, W, m, di, r, kbase, head, qlen, I, lane, held, H);
             }
           }
         }
         __syncwarp();
-        probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, S, H);   // drain before d0s change
+        probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, held, H);   // drain before d0s change
         head = 0;
         qlen = 0;
         __syncwarp();
@@ -458,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5)
           }
         }
         my_probes += __popc(m);
-        push_bits<kSet, kMode>(P, W, m, 0, rr & 63u, kbase, head, qlen, I, lane, S, H);
+        push_bits<kSet, kMode>(P, W, m, 0, rr & 63u, kbase, head, qlen, I, lane, held, H);
         if (find2) {
           r += 32;
         } else if ((wt += W.nparts) >= (len + 1023u) / 1024u) {   // len: the same in every lane
@@ -467,12 +480,13 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5)
         }
       }
       __syncwarp();
-      probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, S, H);
+      probe_batch<kSet, kMode>(P, W, head, qlen, I, lane, held, H);
       __syncwarp();
     }
   }
 
-  if constexpr (kMode == kEmit) stage_close(P.pages, *H, S, lane, DirectProbe{P.tv, P.chunk});
+  if constexpr (kEmits<kMode>)
+    stage_close(P.list, stage_list(), *H, held, lane, DirectProbe{P.tv, P.chunk});
 
   // ---- counters: warp reduce, one atomic per warp ----
 #pragma unroll
@@ -490,8 +504,8 @@ __global__ void __launch_bounds__(kThreads, kSharp ? 3 : kMode == kEmit ? 4 : 5)
 
 // k_peel over items [0, n) of the batch, or for the staged probe over [sl->lo, n).
 struct StageLaunch {
-  u32 lo, sb;
-  StagePages pages;
+  u32 lo;
+  StageRuns list;
   StageChunk* chunk;
 };
 template <bool kSharp, bool kSet, int kMode = kProbe>
@@ -531,10 +545,9 @@ int launch_main(s615_ctx* ctx, const TableView& tv, const s615_batch* b, size_t 
   P.s8 = gated ? 0x7u : 0xFFu;
   if (kMode != kProbe) {
     P.item_lo = sl->lo;
-    P.sb = sl->sb;
-    P.pages = sl->pages;
+    P.list = sl->list;
     P.chunk = sl->chunk;
-    P.work = sl->chunk->work[kMode == kEmit ? 0 : 4];
+    P.work = sl->chunk->work[kEmits<kMode> ? 0 : 5];
   }
   if (n == 0) return S615_OK;
   int grid = grid_blocks;
@@ -604,11 +617,15 @@ int launch_peel(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flag
 }
 
 int launch_stage_peel(s615_ctx* ctx, const TableView& tv, const s615_batch* b, unsigned flags,
-                      cudaStream_t st, bool resolve, u32 lo, u32 hi, u32 sb, const StagePages& pages,
-                      StageChunk* chunk) {
-  const StageLaunch sl{lo, sb, pages, chunk};
-  return resolve ? launch_main<false, false, kResolve>(ctx, tv, b, hi, flags | kFlagNoCount, st, 0, &sl)
-                 : launch_main<false, false, kEmit>(ctx, tv, b, hi, flags, st, 0, &sl);
+                      cudaStream_t st, bool resolve, u32 lo, u32 hi, const StageRuns& list, StageChunk* chunk) {
+  const StageLaunch sl{lo, list, chunk};
+  if (resolve) return launch_main<false, false, kResolve>(ctx, tv, b, hi, flags | kFlagNoCount, st, 0, &sl);
+  if (!tv.eplane) return launch_main<false, false, kEmit>(ctx, tv, b, hi, flags, st, 0, &sl);
+  TableView te = tv;   // the plane that the keys go through first
+  te.plane = tv.eplane;
+  te.plane_lb = 0;
+  te.plane_mask = 1u;
+  return launch_main<false, false, kEmitPlane>(ctx, te, b, hi, flags, st, 0, &sl);
 }
 
 S615_CHECK_TAKE_DEFINE(check_take_peel)

@@ -6,28 +6,35 @@
 // ps.  So a large batch is probed in chunks, in steps that each read a part
 // of the table that stays in L2:
 //
-//   emit     the peel and the gate (k_peel) write each surviving key's hash to
-//            a page of its bucket: the slice of the first third its cell lies in;
-//   stage 1  page by page in bucket order, the low four bits of the first cell
-//            are read from the table's plane (a 17th to a 32nd of a third: 38 MB
-//            at most for N = 76,667) and the key goes on, with them, to a page
-//            by the slice of its second cell;
-//   stage 2  the same with the second and third cells;
-//   stage 3  the third cell's low bits complete the comparison of the low bits;
-//            one key in 16 passes and its cells are read in full.  A key that
-//            the table holds sets its bit in the chunk's Bloom filter;
+//   emit     the peel and the gate (k_peel) append each surviving key's hash to
+//            one of 16 lists (for a table whose one-bit plane fits L2 beside
+//            this: the keys that its bit leaves);
+//   step 0   the keys are sorted by the slice of the first third that their first
+//            cell lies in (a 17th to a 32nd of a third: 38 MB of four-bit cells
+//            at most for N = 76,667);
+//   step 1   slice by slice, four bits of the first cell are read from the plane,
+//            which stays in L2, and the key goes on, with them, by the slice of its
+//            second cell;
+//   step 2   the same with the second and third cells;
+//   step 3   the third cell's bits complete the comparison of the four bits; one
+//            key in 16 passes and its cells are read in full.  A key that the
+//            table holds sets its bit in the chunk's Bloom filter;
 //   resolve  only if the chunk has such a key (a false positive of the filter
 //            included): the peel runs over the chunk once more and probes the
 //            keys whose bit is set, recording hits as ever.
 //
 // The comparison is the probe's own, cut in parts, so hits and counters are the
-// direct probe's.  A key whose bucket has no page left is probed where it is.
+// direct probe's.  A key for which a list or bucket has no room is probed where it is.
 //
 // 12,000 units of the 3.2M class-5 band (20 chunks, 5.2e9 keys): 337 ms probed
-// directly, 250 in stages: emit 74, stage 1 60, stage 2 60, stage 3 42, resolve 15.
-// 6,000 units of the mixed stream at B <= 2M: 29.1 -> 22 ms.  Emit is bound by
-// instruction issue (80% of the slots), the stages by L2 traffic of reads and
-// writes mixed.
+// directly, 198 in stages: emit 55, steps 21, 37, 37 and 35, resolve 15.  6,000 units
+// of the mixed stream at B <= 2M: 29.1 -> 16.5 ms.  Emit is bound by instruction
+// issue, the steps by L2 traffic of reads and writes mixed (the floor of steps 1
+// and 2: 3.5 ps for a plane read and 2.4 for 16 bytes of HBM, of 7 ps a key).
+// Emitting by slice at once, a page per warp and slice, took 74 ms where emit and
+// step 0 take 76, and 12% more on the mixed stream; behind a one-bit plane it took
+// 60 ps a key against 14 (page stores all over HBM and the plane's reads shared
+// the TLB).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,8 +45,7 @@
 namespace s615 {
 
 int launch_stage_peel(s615_ctx* ctx, const TableView& tv, const s615_batch* b, unsigned flags,
-                      cudaStream_t st, bool resolve, u32 lo, u32 hi, u32 sb, const StagePages& pages,
-                      StageChunk* chunk);
+                      cudaStream_t st, bool resolve, u32 lo, u32 hi, const StageRuns& list, StageChunk* chunk);
 
 namespace {
 
@@ -50,24 +56,20 @@ struct StageParams {
   TableView tv;
   const u32* plane;
   u32 sb;
-  StagePages first;   // step 1's input
-  StageRuns in, out;  // the others'
+  u32 bit0;           // the lowest of the four bits that the plane holds
+  StageRuns in, out;
   StageChunk* chunk;
 };
 
 constexpr u32 kPlaneLb = 2;    // 4 bits of each cell, eight cells to a word
 
-// A step's input as units of kUnit entries of one bucket (pages follow one
-// another in a bucket, and a piece is a multiple of a unit): warp-wide state.
-template <int kStep, u32 kUnit>
+// A step's input as units of kUnit entries of one bucket (a piece is a multiple of
+// a unit): warp-wide state.
+template <u32 kUnit>
 struct UnitOrder {
   u32 incl, n, total;
   __device__ __forceinline__ UnitOrder(const StageParams& P, u32 lane) {
-    n = 0;
-    if (kStep == 1 ? lane < P.first.nb : lane < P.in.nb)
-      n = kStep == 1 ? (min(P.first.npages[lane * kStageStride], P.first.cap) + kUnit / kStagePage - 1) /
-                           (kUnit / kStagePage)
-                     : (min(P.in.count[lane * kStageStride], P.in.cap) + kUnit - 1) / kUnit;
+    n = lane < P.in.nb ? (min(P.in.count[lane * kStageStride], P.in.cap) + kUnit - 1) / kUnit : 0u;
     incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -76,18 +78,12 @@ struct UnitOrder {
     }
     total = __shfl_sync(0xFFFFFFFFu, incl, 31);
   }
-  // Unit g < total: its bucket, first entry and length (step 1: its pages'
-  // entries, whatever their fills).
+  // Unit g < total: its bucket, first entry and length.
   __device__ __forceinline__ void at(const StageParams& P, u32 g, u32& b, u64& e, u32& len) const {
     b = __popc(__ballot_sync(0xFFFFFFFFu, incl <= g));   // buckets wholly before unit g
     const u32 i = (g - __shfl_sync(0xFFFFFFFFu, incl - n, b)) * kUnit;
-    if constexpr (kStep == 1) {
-      e = (u64)b * P.first.cap * kStagePage + i;
-      len = min(min(P.first.npages[b * kStageStride], P.first.cap) * kStagePage - i, kUnit);
-    } else {
-      e = P.in.at(b, i);
-      len = min(min(P.in.count[b * kStageStride], P.in.cap) - i, kUnit);
-    }
+    e = P.in.at(b, i);
+    len = min(min(P.in.count[b * kStageStride], P.in.cap) - i, kUnit);
   }
 };
 
@@ -95,28 +91,21 @@ struct UnitOrder {
 template <int kStep>
 __device__ __forceinline__ u64 stage_open(const StageParams& P, u64 e, u32 b, u64& g) {
   const u32 block = (u32)P.tv.block;
-  if constexpr (kStep == 1) {   // entries are the hashes
-    g = e;
-    u64 q;
-    u32 off;
-    split_word(e, block, P.tv.recip, q, off);
-    return off;
-  } else {
-    g = entry_word(e, b, P.sb, block);
-    return (u64)(kStep - 1) * block + ((b << P.sb) | ((u32)(e >> 4) & ((1u << P.sb) - 1u)));
-  }
+  g = entry_word(e, b, P.sb, block);
+  return (u64)(kStep - 1) * block + ((b << P.sb) | ((u32)(e >> 4) & ((1u << P.sb) - 1u)));
 }
 __device__ __forceinline__ u32 plane_bits(u32 w, u64 c) { return w >> (((u32)c & 7u) << kPlaneLb); }
 
-// Steps 1 and 2: look cell kStep - 1 up and send the key on by cell kStep.  The
-// block orders 1,024 keys by bucket in shared memory and appends each bucket's
+// Steps 0 to 2: look cell kStep - 1 up (step 0: nothing) and send the key on by cell
+// kStep.  The block orders 1,024 keys by bucket in shared memory and appends each bucket's
 // run (some 30 to 60 keys) to the bucket.
 //
 // Scattered accesses run at full rate only within the reach of the first-level
 // TLB, which behaves like 128 entries of 2 MB in 8 sets (8 MB of lines in L2 read
 // at 2.8e11/s within 128 MB, at 4.5e10/s spread over 1 GB), so input, output and
-// plane slice are laid out to lie within that (StageRuns).  With a page per
-// warp and bucket, each bucket in a region of its own, a step took 23 ps a key.
+// plane slice are laid out to lie within that (StageRuns).  With the entries in a
+// page per warp and bucket, each bucket in a region of its own, a step took 23 ps a
+// key, against 7.
 //
 // A block always knows its next unit: the queue's answer and the buckets' new
 // ends come back while it works.
@@ -126,30 +115,25 @@ __global__ void __launch_bounds__(kThreads, 5) k_stage(StageParams P) {
   __shared__ unsigned long long s_e[kUnit];
   __shared__ u8 s_b[kUnit];
   __shared__ u32 s_cnt[kStageBuckets], s_off[kStageBuckets], s_dst[kStageBuckets];
-  __shared__ u32 s_fill[kUnit / kStagePage];
   __shared__ u64 s_at;
   __shared__ u32 s_in, s_len, s_total;
   const u32 tid = threadIdx.x, lane = tid & 31;
-  const unsigned long long* in = kStep == 1 ? P.first.e : P.in.e;
+  const unsigned long long* in = P.in.e;
   const u32 block = (u32)P.tv.block, sb = P.sb;
   const u64 recip = P.tv.recip;
-  const UnitOrder<kStep, kUnit> O(P, lane);
+  const UnitOrder<kUnit> O(P, lane);
   // warp 0: unit g's place to shared memory (s_len = 0: no more units)
   auto place = [&](u32 g) {
     u32 b = 0, len = 0;
     u64 e = 0;
     if (g < O.total) O.at(P, g, b, e, len);
-    if (kStep == 1 && lane < kUnit / kStagePage) {
-      const u64 page = e / kStagePage + lane;
-      s_fill[lane] = lane * kStagePage < len ? min(P.first.fill[page], kStagePage) : 0u;
-    }
     if (lane == 0) { s_at = e; s_in = b; s_len = len; }
   };
   u32 next = 0;
   if (tid < 32) {
-    if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+    if (lane == 0) next = atomicAdd(P.chunk->work[kStep + 1], 1u);
     place(__shfl_sync(0xFFFFFFFFu, next, 0));
-    if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+    if (lane == 0) next = atomicAdd(P.chunk->work[kStep + 1], 1u);
     s_cnt[lane] = 0;
   }
   for (;;) {
@@ -162,24 +146,29 @@ __global__ void __launch_bounds__(kThreads, 5) k_stage(StageParams P) {
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
       const u32 i = (u32)k * kThreads + tid;
-      const bool on = kStep == 1 ? i % kStagePage < s_fill[i / kStagePage] : i < len;
+      const bool on = i < len;
       g[k] = on ? (u64)__ldcs(src + i) : 0;
       act |= (u32)on << k;
     }
     // the plane's answers come back while the next words are worked out
+    if constexpr (kStep > 0) {
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const u32 e = (u32)g[k];
-      const u64 c = stage_open<kStep>(P, g[k], ib, g[k]);
-      x[k] = (e & 15u) | ((u32)c & 7u) << 6;   // low bits so far | 4 * (cell % 8)
-      const bool on = ((act >> k) & 1u) && S615_CHECK(c < 3 * (u64)block, kChkCell);
-      w[k] = on ? __ldcg(P.plane + (c >> (5 - kPlaneLb))) : 0u;
+      for (int k = 0; k < kPer; ++k) {
+        const u32 e = (u32)g[k];
+        const u64 c = stage_open<kStep>(P, g[k], ib, g[k]);
+        x[k] = (e & 15u) | ((u32)c & 7u) << 6;   // low bits so far | 4 * (cell % 8)
+        const bool on = ((act >> k) & 1u) && S615_CHECK(c < 3 * (u64)block, kChkCell);
+        w[k] = on ? __ldcg(P.plane + (c >> (5 - kPlaneLb))) : 0u;
+      }
+    } else {   // the hash's own bits to begin with
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) { x[k] = (u32)(g[k] >> P.bit0) & 15u; w[k] = 0; }
     }
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
       u64 q;
       u32 off;
-      split_word(cell_word<kStep>(hash_of_word<kStep - 1>(g[k])), block, recip, q, off);
+      split_word(cell_word<kStep>(hash_of_word<kStep ? kStep - 1 : 0>(g[k])), block, recip, q, off);
       g[k] = pack_entry(q, off, sb, 0);
       const u32 b = off >> sb;
       at[k] = ((act >> k) & 1u) ? b | (atomicAdd(&s_cnt[b], 1u) << 5) : kNone;
@@ -212,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_stage(StageParams P) {
       }
     if (tid < 32) {
       place(__shfl_sync(0xFFFFFFFFu, next, 0));
-      if (lane == 0) next = atomicAdd(P.chunk->work[kStep], 1u);
+      if (lane == 0) next = atomicAdd(P.chunk->work[kStep + 1], 1u);
       s_dst[lane] = base - off0;   // entry i of the tile goes to place s_dst + i
     }
     __syncthreads();
@@ -221,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_stage(StageParams P) {
       const u32 b = s_b[pos], i = s_dst[b] + pos;
       const u64 e = s_e[pos];
       if (i < P.out.cap) {
-        P.out.e[P.out.at(b, i)] = e;
+        __stcs(P.out.e + P.out.at(b, i), (unsigned long long)e);
       } else {   // no room left in the bucket: probed here
         const u64 h = hash_of_word<kStep>(entry_word(e, b, sb, block));
         if (contains_hash<false>(P.tv, h)) stage_positive(P.chunk, h);
@@ -243,9 +232,9 @@ __global__ void __launch_bounds__(kThreads) k_stage_last(StageParams P) {
   const u32 lane = threadIdx.x & 31;
   u32 lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-  const UnitOrder<3, kTake> O(P, lane);
+  const UnitOrder<kTake> O(P, lane);
   u32 next = 0, held = 0;
-  if (lane == 0) next = atomicAdd(P.chunk->work[3], 1u);
+  if (lane == 0) next = atomicAdd(P.chunk->work[4], 1u);
   auto probe = [&](u32 first, u32 n) {   // entries [first, first + n), n <= 32: words of cell 2
     if (lane < n) {
       const u64 h = hash_of_word<2>(agree[first + lane]);
@@ -255,7 +244,7 @@ __global__ void __launch_bounds__(kThreads) k_stage_last(StageParams P) {
   for (;;) {
     const u32 unit = __shfl_sync(0xFFFFFFFFu, next, 0);
     if (unit >= O.total) break;
-    if (lane == 0) next = atomicAdd(P.chunk->work[3], 1u);
+    if (lane == 0) next = atomicAdd(P.chunk->work[4], 1u);
     u32 b, len;
     u64 at;
     O.at(P, unit, b, at, len);
@@ -305,36 +294,33 @@ int launch_stage(s615_ctx* ctx, K kernel, const StageParams& P, cudaStream_t st)
   return S615_OK;
 }
 
-// Most warps of any of the kernels that write pages (each may leave a page
-// part-filled in every bucket).
-u64 stage_warps(const s615_ctx* ctx) { return (u64)ctx->num_sms * 64; }
-
 // Keys per chunk: enough that reading the plane once per chunk and the ends of
-// six launches are small beside it, few enough that most chunks of a search hold
+// seven launches are small beside it, few enough that most chunks of a search hold
 // no key of the table (about one in 1e9) and skip the resolve pass.
 constexpr u64 kMaxChunkKeys = 1ull << 28, kMinChunkKeys = 1ull << 26;
-// The least keys for which the stages pay: below, six launches and part-filled
-// pages cost more than the scattered reads.  Direct / staged, ms, class-5 units:
+// The least keys for which the stages pay: below, seven launches and their ends
+// cost more than the scattered reads.  Direct / staged, ms, class-5 units:
 // 1e7 keys 0.74 / 0.69 (N = 42,000), 0.55 / 0.60 (31,000); 2e7 1.47 / 1.07 and
 // 0.99 / 0.91; 2.4e7 1.72 / 1.44 (76,667), but 1.64 / 1.74 with a key of the table
 // among them, when the resolve pass runs; 4.4e7 2.93 / 2.22; 1e8 7.2 / 4.4.
 constexpr double kMinKeys = 2.5e7;
 
-// Two spaces in turn: the emitted pages, stage 1's runs, stage 2's in the
-// pages' place.
+// Two spaces in turn: the emitted keys, then by first cell, by second (in the first
+// space again), by third.
 struct Layout {
-  u32 nb = 0, pages = 0, entries = 0;   // per bucket: pages emitted, entries of a run
+  u32 nb = 0, list = 0, entries = 0;   // room of an emitted list and of a bucket
   size_t first = 0, second = 0, bytes = 0;
 };
-Layout layout_for(const s615_ctx* ctx, u64 keys, u32 nb) {
+Layout layout_for(u64 keys, u32 nb) {
   Layout L;
   L.nb = nb;
-  const u64 each = (keys + keys / 8) / nb;
-  L.pages = (u32)(each / kStagePage + stage_warps(ctx));
-  L.entries = (u32)((each >> kStagePieceLog2) + 1) << kStagePieceLog2;
+  const auto room = [&](u32 parts) {
+    return (u32)((((keys + keys / 8) / parts >> kStagePieceLog2) + 1) << kStagePieceLog2);
+  };
+  L.list = room(kStageLists);
+  L.entries = room(nb);
   L.second = (size_t)nb * L.entries * 8;
-  L.first = std::max(L.second, (size_t)nb * L.pages * (kStagePage * 8 + 4));
-  L.first = (L.first + 255) / 256 * 256;
+  L.first = std::max(L.second, (size_t)kStageLists * L.list * 8);
   L.bytes = (sizeof(StageChunk) + 255) / 256 * 256 + L.first + L.second;
   return L;
 }
@@ -366,19 +352,20 @@ int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned fl
     cudaGetLastError();
     return S615_OK;
   }
+  if (tv.eplane) est /= 2;   // the keys that its bit leaves
   std::lock_guard<std::mutex> lock(ctx->stage.mu);
   StageSpace& w = ctx->stage;
   // chunks of at most kMaxChunkKeys keys, smaller when HBM is short
   u64 keys = (u64)std::min<double>(est * 1.05, (double)kMaxChunkKeys);
   const u32 sb = stage_shift(tv.block);
   const u32 nb = (u32)((tv.block + (1ull << sb) - 1) >> sb);
-  Layout L = layout_for(ctx, keys, nb);
+  Layout L = layout_for(keys, nb);
   if (L.bytes > w.bytes) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
     const size_t used = ctx->used.load();
     const size_t room = w.bytes + std::min(free_b, ctx->budget > used ? ctx->budget - used : 0) / 4;
-    while (L.bytes > room && keys > kMinChunkKeys) L = layout_for(ctx, keys = std::max(keys / 2, kMinChunkKeys), nb);
+    while (L.bytes > room && keys > kMinChunkKeys) L = layout_for(keys = std::max(keys / 2, kMinChunkKeys), nb);
     if (L.bytes > w.bytes) {
       if (L.bytes > room) return S615_OK;
       stage_release(ctx);
@@ -395,29 +382,31 @@ int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned fl
   char* at = static_cast<char*>(w.p) + (sizeof(StageChunk) + 255) / 256 * 256;
   auto* first = reinterpret_cast<unsigned long long*>(at);
   auto* second = reinterpret_cast<unsigned long long*>(at + L.first);
-  const StagePages pages{first, reinterpret_cast<u32*>(first + (size_t)nb * L.pages * kStagePage),
-                         chunk->count[0], nb, L.pages};
+  const StageRuns list{first, chunk->count[0], kStageLists, L.list};
   const u64 chunks = std::max<u64>(1, (u64)(est / (double)keys + 0.999));
   int s = S615_OK;
   for (u64 c = 0; c < chunks && !s; ++c) {
     const u32 lo = (u32)(b->n_main * c / chunks), hi = (u32)(b->n_main * (c + 1) / chunks);
     if (lo == hi) continue;
     if (cudaMemsetAsync(chunk, 0, sizeof(StageChunk), st) != cudaSuccess) { s = S615_E_DEVICE; break; }
-    if ((s = launch_stage_peel(ctx, tv, b, flags, st, false, lo, hi, sb, pages, chunk))) break;
+    if ((s = launch_stage_peel(ctx, tv, b, flags, st, false, lo, hi, list, chunk))) break;
     StageParams P{};
     P.tv = tv;
     P.plane = tv.splane;
+    P.bit0 = tv.eplane ? 1u : 0u;
     P.sb = sb;
     P.chunk = chunk;
-    P.first = pages;
-    P.out = StageRuns{second, chunk->count[1], nb, L.entries};
-    if ((s = launch_stage(ctx, k_stage<1>, P, st))) break;
-    P.in = P.out;
-    P.out = StageRuns{first, chunk->count[2], nb, L.entries};
-    if ((s = launch_stage(ctx, k_stage<2>, P, st))) break;
+    P.out = list;
+    for (int k = 0; k < 3 && !s; ++k) {
+      P.in = P.out;
+      P.out = StageRuns{k == 1 ? first : second, chunk->count[k + 1], nb, L.entries};
+      s = k == 0 ? launch_stage(ctx, k_stage<0>, P, st)
+        : k == 1 ? launch_stage(ctx, k_stage<1>, P, st) : launch_stage(ctx, k_stage<2>, P, st);
+    }
+    if (s) break;
     P.in = P.out;
     if ((s = launch_stage(ctx, k_stage_last, P, st))) break;
-    s = launch_stage_peel(ctx, tv, b, flags, st, true, lo, hi, sb, pages, chunk);
+    s = launch_stage_peel(ctx, tv, b, flags, st, true, lo, hi, list, chunk);
   }
   cudaEventRecord(w.last, st);
   return s;

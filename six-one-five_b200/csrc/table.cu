@@ -61,9 +61,9 @@ __global__ void k_pack(const Cell* __restrict__ wide, u64 m, u32 r,
   }
 }
 
-// One thread per 32-bit plane word: the low 2^lb bits of its 32 >> lb cells.
+// One thread per 32-bit plane word: 2^lb bits, from bit `shift` on, of its 32 >> lb cells.
 __global__ void k_plane(const void* __restrict__ cells, u32 layout, u32 cell_bytes, u32 r, u64 m,
-                        u32 lb, u32* __restrict__ plane, u64 n_words) {
+                        u32 lb, u32 shift, u32* __restrict__ plane, u64 n_words) {
   const u32 per = 32u >> lb, bits = 1u << lb;
   const u32 mask = (u32)((1ull << bits) - 1);
   for (u64 w = blockIdx.x * (u64)blockDim.x + threadIdx.x; w < n_words;
@@ -71,7 +71,7 @@ __global__ void k_plane(const void* __restrict__ cells, u32 layout, u32 cell_byt
     const u64 c0 = w * per;
     u32 word = 0;
     for (u32 k = 0; k < per && c0 + k < m; ++k)
-      word |= ((u32)load_cell_at(cells, layout, cell_bytes, r, fp_mask(r), c0 + k) & mask) << (k * bits);
+      word |= ((u32)(load_cell_at(cells, layout, cell_bytes, r, fp_mask(r), c0 + k) >> shift) & mask) << (k * bits);
     plane[w] = word;
   }
 }
@@ -128,6 +128,7 @@ TableView view_of(const DevTable& t) {
   v.cell_bytes = (u32)t.cell_bytes;
   v.plane = static_cast<const u32*>(t.d_plane);
   v.splane = static_cast<const u32*>(t.d_splane);
+  v.eplane = static_cast<const u32*>(t.d_eplane);
   v.plane_bytes = t.plane_bytes;
   v.plane_lb = t.plane_lb;
   v.plane_mask = (u32)((1ull << (1u << t.plane_lb)) - 1);
@@ -135,12 +136,14 @@ TableView view_of(const DevTable& t) {
   return v;
 }
 
-// The low 2^lb bits of t's cells; *p stays null when there is no room.
-static int make_plane(s615_ctx* ctx, const DevTable& t, int lb, cudaStream_t st, void** p, size_t* bytes) {
+// 2^lb bits of t's cells, from bit `shift` on; *p stays null when there is no room.
+static int make_plane(s615_ctx* ctx, const DevTable& t, int lb, u32 shift, cudaStream_t st, void** p,
+                      size_t* bytes) {
   const u64 m = t.hdr.m_cells, per = 32u >> lb, words = (m + per - 1) / per;
   if (dev_alloc_once(ctx, p, words * sizeof(u32))) return S615_OK;
   k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
-                                                     t.hdr.r, m, (u32)lb, static_cast<u32*>(*p), words);
+                                                     t.hdr.r, m, (u32)lb, shift,
+                                                     static_cast<u32*>(*p), words);
   ctx->launches++;
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -164,11 +167,17 @@ static int make_plane(s615_ctx* ctx, const DevTable& t, int lb, cudaStream_t st,
 // bit) 63.1 / 42.9, 36,000 (1 bit) 63.2 / 47.5; (6,1,7), N = 10,476 (8 bits) 54.7 /
 // 14.  Three reads of a 64 MB plane are 10.5 ps.
 constexpr double kPlaneMaxMB = 112;
-// The staged probe takes 34 to 37 ps a key, whatever the table (N = 20,000 to
-// 76,667, 2e8 keys), so tables whose probe costs more by this count get its plane
-// as well, for their large batches: N = 28,000 (1 bit) 42.6 -> 34.3 ps, 36,000 48.0
-// -> 36.0, 48,000 63.1 -> 35.8; N = 24,000 (2 bits, 30.7 ps) would lose.
-constexpr double kStagedPs = 38;
+// The staged probe takes 33 to 36 ps a key whatever the table, 28 of them after the
+// sieve, so tables whose probe costs more than kStagedFrom by this count get its
+// planes as well, for their large batches: four bits, and if it is small enough to
+// be read at the full rate beside the sieve (58 MB: 14 ps a key; 70 MB 21, 84 MB
+// 27), a plane of one bit that keeps half of the keys out of the stages.  2e8
+// class-5 keys, ps a key probed directly / in stages: N = 22,000 28.0 / 28.6 (left as
+// it is), 24,000 30.8 / 28.3, 26,500 34.7 / 27.6, 28,000 41.5 / 28.6, 29,500 (four bits
+// only from here) 42.7 / 33.2, 31,000 43.0 / 32.9, 36,000 47.9 / 35.3, 42,000 61.5 / 34.8,
+// 76,667 63.8 / 36.3.
+constexpr double kStagedFrom = 29;
+constexpr u64 kEPlaneMax = 60ull << 20;
 int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   const u64 m = t.hdr.m_cells;
   if (!t.d_cells || t.hdr.n_keys == 0 || m < 3) return S615_OK;
@@ -183,18 +192,23 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
     if (mb <= kPlaneMaxMB && ps < best) { best = ps; lb = k; }
   }
   if (lb >= 0) {
-    if (const int s = make_plane(ctx, t, lb, st, &t.d_plane, &t.plane_bytes)) return s;
+    if (const int s = make_plane(ctx, t, lb, 0, st, &t.d_plane, &t.plane_bytes)) return s;
     t.plane_lb = (u32)lb;
   }
   // The staged probe's plane, when its slices (staged.cuh) fit L2.  Below 16 bits
   // the filter's own false positives (2^-r of the keys) fill the chunk's Bloom
   // filter, and the last pass would probe most keys again.
-  if ((t.d_plane ? best : cell_ps) < kStagedPs || t.hdr.r < 16 || m / 2 / 3 / 16 > kStageSlice)
+  if ((t.d_plane ? best : cell_ps) < kStagedFrom || t.bytes < ((size_t)1 << 28) || t.hdr.r < 16 ||
+      m / 2 / 3 / 16 > kStageSlice)
     return S615_OK;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
   if (4 * (m / 2) > free_b) return S615_OK;   // room that a search will want
-  return make_plane(ctx, t, 2, st, &t.d_splane, &t.splane_bytes);
+  if (m / 8 <= kEPlaneMax) {
+    if (t.d_plane && lb == 0) t.d_eplane = t.d_plane;
+    else if (const int s = make_plane(ctx, t, 0, 0, st, &t.d_eplane, &t.eplane_bytes)) return s;
+  }
+  return make_plane(ctx, t, 2, t.d_eplane ? 1u : 0u, st, &t.d_splane, &t.splane_bytes);
 }
 
 int launch_xor_query(s615_ctx* ctx, const TableView& tv, const u64* d_keys, size_t n,

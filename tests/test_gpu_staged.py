@@ -66,15 +66,24 @@ def test_class5(staged_table):
         assert ((got[:, 0] == len(units) + j) & (got[:, 4] == np.uint64(p.fp))).any()
 
 
-def test_table_with_both_planes():
-    """N = 34,000: a 1-bit plane for the small batches, 4 bits for the stages."""
+@pytest.mark.parametrize("N,bits,first,n", [(34000, 1, 0, 1501), (28000, 1, 1, 2000),
+                                            (25001, 2, 1, 2600)])
+def test_table_with_planes_of_its_own(N, bits, first, n):
+    """A table with a plane of 1 or 2 bits: the keys go through one of one bit, if it is
+    small enough (perhaps that plane), into the stages, which compare the next four."""
     with s615.Engine(0) as eng:
-        tid = eng.build_table(34000, 20)
+        tid = eng.build_table(N, 20)
         info = eng.table_info(tid)
         m = info.hdr.m_cells
-        assert info.device_bytes == 4 * m + (m + 31) // 32 * 4 + (m + 7) // 8 * 4
-        arr, n = W.unit_array(W.cls5_units(1425000, 1425900)[:1501], [], 34000)
-        check(eng, tid, arr, n, 100)
+        plane = lambda k: (m + 32 // k - 1) // (32 // k) * 4 if k else 0
+        own = plane(first) if first != bits else 0
+        assert info.device_bytes == 4 * m + plane(bits) + own + plane(4)
+        B = 42 * N - 3000
+        plants = W.plants(9, 4, B - 90000, B, N)
+        arr, k = W.unit_array(W.cls5_units(B, B + 2900)[:n], plants, N)
+        got = check(eng, tid, arr, k, 100)
+        for j, p in enumerate(plants):
+            assert ((got[:, 0] == k - len(plants) + j) & (got[:, 4] == np.uint64(p.fp))).any()
 
 
 def test_no_gate(staged_table):
