@@ -71,7 +71,7 @@ def parse():
     ap.add_argument("--seconds", type=float, default=10.0, help="serve: seconds of arrivals")
     ap.add_argument("--slots", type=int, default=2, help="serve: batches in flight")
     ap.add_argument("--no-l2-window", action="store_true",
-                    help="cls5: time the pass without the peel's L2-persisting access window")
+                    help="cls5: pass S615_F_NO_L2_WINDOW (no effect: no launch carries a window)")
     ap.add_argument("--reference-gpu", type=int, default=15536,
                     help="cls5: run the reference's fourcore_cls5_gpu_v4 on K evenly spaced band "
                          "units (default: a tenth of the band; 0: the whole band; -1: skip)")
@@ -765,7 +765,7 @@ def run_cfg1(args, rank, world, local, dist):
     """--workload cfg1: the small CPU-runnable configuration -- every class-5
     unit of B in [1000, 30000] (725) plus 8 plants against an N = 715, r = 48
     table built on the device (1.9 MB) -- timed with and without the peel's
-    L2-persisting access window, and the oracle on the host cores beside it."""
+    S615_F_NO_L2_WINDOW (which has no effect any more), and the oracle on the host cores beside it."""
     import numpy as np
     import torch
 
@@ -1420,11 +1420,11 @@ def main():
             "%.3e" % roof["random_access"]["ceiling_reads_per_s"]
             if roof["random_access"]["ceiling_reads_per_s"] else "n/a",
             roof["random_access"]["frac"]))
-    # DRAM bytes the probe moves: each cell read misses L2 and fills one 64-byte
-    # line (ld.global.cg.L2::64B; a one-pass ncu capture of the full pass
-    # measured 191.7 B per post-gate probe); against the same copy peak
-    dram = 3 * 64 * ctr.probes / dur_s / 1e9
-    roof["dram_fills"] = {"bytes_per_cell_read": 64, "achieved": round(dram, 1), "peak": peak,
+    # DRAM bytes the staged probe moves per post-gate key: eight passes of its 8-byte
+    # entry (written and read between the steps) and, for one key in 16, three 64-byte
+    # fills of its cells; against the same copy peak
+    dram = 76 * ctr.probes / dur_s / 1e9
+    roof["dram_fills"] = {"bytes_per_key": 76, "achieved": round(dram, 1), "peak": peak,
                           "unit": "GB/s", "frac": round(dram / peak, 4)}
 
     # plain per-unit-launch form on a bounded sample of the same band
@@ -1534,7 +1534,7 @@ def main():
                    "shards": args.shards,
                    "units_per_rank": n, "N": N, "r": args.r,
                    "l2": "inputs larger than L2 (table %.1f GB)" % (eng.table_info(tid).device_bytes / 1e9),
-                   "l2_window": not args.no_l2_window,
+                   "l2_window": False,
                    "parallelism": (f"shard-split x{world}: each rank holds {args.shards // world}+ of "
                                    f"{args.shards} shards and runs the whole band" if split
                                    else f"replicas-by-band x{world}")},

@@ -61,7 +61,7 @@ typedef struct s615_table_info {
   s615_header hdr;
   int layout;             /* S615_LAYOUT_PACKED or _WIDE */
   int cell_bytes;         /* 0 for PACKED, else 4 or 8 */
-  uint64_t device_bytes;  /* HBM held by the table */
+  uint64_t device_bytes;  /* HBM held by the table: its cells and their planes */
 } s615_table_info;
 
 /* Unit record.  cls 5: the 2-D (e,d) peel; cls 2, 3, 4: one free term d
@@ -368,8 +368,11 @@ int s615_cls5_run(s615_ctx* ctx, int table_id, const s615_unit* units, size_t n,
                   unsigned flags, s615_hit* hits, size_t hit_cap, size_t* n_hits,
                   s615_counters* counters);
 /* Device-resident form: the units are packed and uploaded once
- * (s615_prepare); each s615_run_batch is one launch on the caller's stream
- * (NULL = the context's stream); results stay on the device until
+ * (s615_prepare); each s615_run_batch is one or two launches on the caller's
+ * stream (NULL = the context's stream), or for a large batch against a table
+ * past L2 a sequence of launches there (with a space of up to a quarter of the
+ * free HBM, kept and given back as s615_run's buffers are; not while the stream
+ * is being captured); results stay on the device until
  * s615_batch_results.  s615_batch_free first waits for the batch's last
  * s615_run_batch to finish (it may be called right after the launch, with no
  * sync), then hands the batch's device buffers to a pool on the context (up to
@@ -393,8 +396,10 @@ int s615_prepare_band(s615_ctx* ctx, uint64_t B_lo, uint64_t B_hi, s615_batch** 
 /* The (cls, B, u) records of a batch's units, in batch order (to verify or
  * report the hits of a device-generated batch). */
 int s615_batch_units(s615_ctx* ctx, const s615_batch* b, s615_unit* out, size_t cap, size_t* n);
-/* What s615_prepare copied to the device: unit records, work items and the
- * host-to-device bytes of both (no counterpart in the reference). */
+/* A batch's unit records and work items, and the host-to-device bytes that
+ * s615_prepare copied for them: both, or the caller's 72-byte records where the
+ * device makes them (no counterpart in the reference).  A band's: its records'
+ * and items' size. */
 int s615_batch_size(const s615_batch* b, size_t* n_units, size_t* n_items, size_t* h2d_bytes);
 
 /* No counterpart in the reference.  s615_cls5_run for callers that cannot
