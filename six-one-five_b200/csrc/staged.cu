@@ -29,8 +29,10 @@
 // 12,000 units of the 3.2M class-5 band (20 chunks, 5.2e9 keys): 337 ms probed
 // directly, 198 in stages: emit 55, steps 21, 37, 37 and 35, resolve 15.  6,000 units
 // of the mixed stream at B <= 2M: 29.1 -> 16.5 ms.  Emit is bound by instruction
-// issue, the steps by L2 traffic of reads and writes mixed (the floor of steps 1
-// and 2: 3.5 ps for a plane read and 2.4 for 16 bytes of HBM, of 7 ps a key).
+// issue, step 3 by the scattered reads of one key in 16, steps 1 and 2 by the chain
+// load, plane read, order, store between block barriers (7 ps a key; the floor is
+// 3.5 for a plane read and 2.4 for 16 bytes of HBM; 6 blocks of 256 or 10 of 128
+// threads a SM: the same, 128 threads with 8 keys each: 230 ms a pass for 200).
 // Emitting by slice at once, a page per warp and slice, took 74 ms where emit and
 // step 0 take 76, and 12% more on the mixed stream; behind a one-bit plane it took
 // 60 ps a key against 14 (page stores all over HBM and the plane's reads shared
