@@ -938,7 +938,7 @@ static u32 tune_bucket(size_t n) {
 // caller (or the serving loop) that prepares a batch while another runs would
 // lose that overlap: then the host does the work.
 static bool device_idle(s615_ctx* ctx) {
-  if (ctx->server) return false;
+  if (serving(ctx)) return false;
   if (!ctx->last_run) return true;
   const cudaError_t e = cudaEventQuery(ctx->last_run);
   if (e != cudaSuccess && e != cudaErrorNotReady) cudaGetLastError();

@@ -282,6 +282,7 @@ int cuda_status(cudaError_t e);
 // Serving: true when a request loop owns the context and the caller is not
 // its worker thread (calls that allocate or launch then return S615_E_BUSY).
 bool serving_blocks(s615_ctx* ctx);
+bool serving(const s615_ctx* ctx);    // true while a request loop owns the context
 void server_destroy(s615_ctx* ctx);   // stops the loop (draining it) and frees it
 
 // Host staging (grow-only; nullptr if even a pageable buffer cannot be had).

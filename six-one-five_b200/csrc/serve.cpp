@@ -268,7 +268,10 @@ struct Server {
   }
 };
 
-bool serving_blocks(s615_ctx* ctx) { return ctx && ctx->server && ctx->server->running && !t_worker; }
+// s615_serve_stop leaves the Server (its results stay readable): running says
+// whether its worker has the context.
+bool serving(const s615_ctx* ctx) { return ctx && ctx->server && ctx->server->running; }
+bool serving_blocks(s615_ctx* ctx) { return serving(ctx) && !t_worker; }
 
 void server_destroy(s615_ctx* ctx) {
   if (!ctx || !ctx->server) return;
