@@ -1210,6 +1210,7 @@ int s615_batch_free(s615_ctx* ctx, s615_batch* b) {
 int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* stream) {
   NvtxRange nvtx("s615_run_batch");
   if (!ctx || !b) return S615_E_ARG;
+  flags &= ~kInternalFlags;   // a caller's stray bits mean nothing
   DevTable* t = find_table(ctx, id);
   if (!t) return S615_E_NOTABLE;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;

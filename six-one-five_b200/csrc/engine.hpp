@@ -122,6 +122,9 @@ constexpr u64 kProbeGroupBytes = 56ull << 30;
 constexpr unsigned kFlagNoCount = 1u << 30;
 // Internal launch flag: the classes 2-5 items have been run already.
 constexpr unsigned kFlagNoMain = 1u << 29;
+// The two share the word of the public flags: s615_run_batch, which every
+// caller's flags pass through, takes them out.
+constexpr unsigned kInternalFlags = kFlagNoCount | kFlagNoMain;
 
 // Kernel-facing view of a table (or of a shard set: shards > 1, parts).
 struct TableView {
