@@ -1216,18 +1216,20 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   const TableView tv = view_of(*t);
   // after the launches: an event that s615_batch_free waits on before the
-  // batch's buffers go to the pool (the caller may free without a sync)
+  // batch's buffers go to the pool (the caller may free without a sync).  Not in
+  // a capture: nothing has run then, and waiting for an event that was last recorded
+  // in one is an error (the caller frees the batch once its graph's replays are done).
   auto mark_done = [&]() {
-    if (!b->done && cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      b->done = nullptr;
-    }
-    if (b->done) cudaEventRecord(b->done, st);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
       cudaGetLastError();
       return;
     }
+    if (!b->done && cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      b->done = nullptr;
+    }
+    if (b->done) cudaEventRecord(b->done, st);
     if (!ctx->last_run && cudaEventCreateWithFlags(&ctx->last_run, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       ctx->last_run = nullptr;
