@@ -61,7 +61,8 @@ typedef struct s615_table_info {
   s615_header hdr;
   int layout;             /* S615_LAYOUT_PACKED or _WIDE */
   int cell_bytes;         /* 0 for PACKED, else 4 or 8 */
-  uint64_t device_bytes;  /* HBM held by the table: its cells and their planes */
+  uint64_t device_bytes;  /* HBM held by the table: its cells and the planes made of them
+                             (which are given back when an allocation needs their room) */
 } s615_table_info;
 
 /* Unit record.  cls 5: the 2-D (e,d) peel; cls 2, 3, 4: one free term d

@@ -48,11 +48,23 @@ int dev_alloc_once(s615_ctx* ctx, void** p, size_t bytes) {
   return S615_E_OOM;
 }
 
-// A failed allocation gives back s615_run's kept batch, if it holds one that
-// no run is using, and tries once more.
+// A failed allocation gives back what the context keeps for later runs (s615_run's
+// batch, if no run is using it, freed batches' buffers, the staged probe's space), and
+// then the tables' planes, and tries again after each.
 int dev_alloc(s615_ctx* ctx, void** p, size_t bytes) {
   if (dev_alloc_once(ctx, p, bytes) == S615_OK) return S615_OK;
-  return release_run_batch(ctx) ? dev_alloc_once(ctx, p, bytes) : S615_E_OOM;
+  if (release_run_batch(ctx) && dev_alloc_once(ctx, p, bytes) == S615_OK) return S615_OK;
+  return release_planes(ctx) ? dev_alloc_once(ctx, p, bytes) : S615_E_OOM;
+}
+
+size_t hbm_room(const s615_ctx* ctx) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const size_t used = ctx->used.load();
+  return std::min(free_b, ctx->budget > used ? ctx->budget - used : 0);
 }
 
 void dev_free(s615_ctx* ctx, void* p, size_t bytes) {
@@ -171,6 +183,31 @@ bool gate_product_matches();
 
 namespace {
 
+void free_planes(s615_ctx* ctx, DevTable& t) {
+  dev_free(ctx, t.d_plane, t.plane_bytes);
+  dev_free(ctx, t.d_splane, t.splane_bytes);
+  if (t.eplane_bytes) dev_free(ctx, t.d_eplane, t.eplane_bytes);
+  t.d_plane = t.d_splane = t.d_eplane = nullptr;
+  t.plane_bytes = t.splane_bytes = t.eplane_bytes = 0;
+}
+
+size_t plane_bytes(const DevTable& t) { return t.plane_bytes + t.splane_bytes + t.eplane_bytes; }
+
+// What release_planes could give back now (the caller holds plane_mu).
+size_t spare_planes(const s615_ctx* ctx) {
+  size_t b = 0;
+  for (const auto& kv : ctx->tables)
+    if (!kv.second.planes_captured) b += plane_bytes(kv.second);
+  return ctx->plane_users ? 0 : b;
+}
+
+// A launch on a stream that is being captured leaves the planes' addresses in a graph.
+void note_capture(DevTable& t, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusNone) t.planes_captured = true;
+}
+
 void free_table(s615_ctx* ctx, DevTable& t) {
   for (DevTable& p : t.parts) free_table(ctx, p);
   t.parts.clear();
@@ -179,16 +216,12 @@ void free_table(s615_ctx* ctx, DevTable& t) {
   dev_free(ctx, t.d_cells, t.bytes);
   t.d_cells = nullptr;
   t.bytes = 0;
-  dev_free(ctx, t.d_plane, t.plane_bytes);
-  dev_free(ctx, t.d_splane, t.splane_bytes);
-  if (t.eplane_bytes) dev_free(ctx, t.d_eplane, t.eplane_bytes);
-  t.d_plane = t.d_splane = t.d_eplane = nullptr;
-  t.plane_bytes = t.splane_bytes = t.eplane_bytes = 0;
+  free_planes(ctx, t);
 }
 
 // Device bytes of a table or of every shard of a set.
 size_t table_bytes(const DevTable& t) {
-  size_t b = t.bytes + t.plane_bytes + t.splane_bytes + t.eplane_bytes;
+  size_t b = t.bytes + plane_bytes(t);
   for (const DevTable& p : t.parts) b += p.bytes;
   return b;
 }
@@ -250,11 +283,15 @@ int pick_layout(s615_ctx* ctx, int want, u64 m, u32 r, int* cell_bytes) {
   if (want == S615_LAYOUT_PACKED) { *cell_bytes = 0; return S615_LAYOUT_PACKED; }
   if (want == S615_LAYOUT_WIDE) return S615_LAYOUT_WIDE;
   release_run_batch(ctx);   // a table needs the room more than s615_run's kept buffers
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
   const size_t wide = m * (size_t)(*cell_bytes) + packed_bytes(m, r) + ((size_t)4 << 30);
-  const size_t room = std::min(free_b, ctx->budget ? ctx->budget - std::min(ctx->budget, ctx->used.load()) : free_b);
+  const size_t room = hbm_room(ctx);
   if (wide <= room) return S615_LAYOUT_WIDE;
+  size_t spare = 0;
+  {
+    std::lock_guard<std::mutex> lock(ctx->plane_mu);
+    spare = spare_planes(ctx);
+  }
+  if (wide <= room + spare && release_planes(ctx) && wide <= hbm_room(ctx)) return S615_LAYOUT_WIDE;
   *cell_bytes = 0;
   return S615_LAYOUT_PACKED;
 }
@@ -283,10 +320,23 @@ int finish_upload(s615_ctx* ctx, DevTable& t, void* d_packed, size_t packed_allo
 
 }  // namespace
 
-// ======================================================================= ABI
 namespace s615 {
 
+bool release_planes(s615_ctx* ctx) {
+  std::lock_guard<std::mutex> lock(ctx->plane_mu);
+  if (!spare_planes(ctx)) return false;
+  if (cudaDeviceSynchronize() != cudaSuccess) {   // what was launched with them has ended
+    cudaGetLastError();
+    return false;
+  }
+  for (auto& kv : ctx->tables)
+    if (!kv.second.planes_captured) free_planes(ctx, kv.second);
+  return true;
+}
+
 }  // namespace s615
+
+// ======================================================================= ABI
 
 extern "C" {
 
@@ -422,8 +472,10 @@ int s615_xor_query_dev(s615_ctx* ctx, int id, const uint64_t* d_keys, size_t n, 
   if (!ctx) return S615_E_ARG;
   DevTable* t = find_table(ctx, id);
   if (!t) return S615_E_NOTABLE;
-  return launch_xor_query(ctx, view_of(*t), d_keys, n, d_out,
-                          stream ? static_cast<cudaStream_t>(stream) : ctx->stream);
+  cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  const PlaneUse use(ctx);
+  note_capture(*t, st);
+  return launch_xor_query(ctx, view_of(*t), d_keys, n, d_out, st);
 }
 
 int s615_xor_query(s615_ctx* ctx, int id, const uint64_t* keys, size_t n, uint8_t* out) {
@@ -437,6 +489,7 @@ int s615_xor_query(s615_ctx* ctx, int id, const uint64_t* keys, size_t n, uint8_
   int s = dev_alloc(ctx, &dk, chunk * 8);
   if (s) return s;
   if ((s = dev_alloc(ctx, &dout, chunk))) { dev_free(ctx, dk, chunk * 8); return s; }
+  const PlaneUse use(ctx);
   const TableView tv = view_of(*t);
   for (size_t off = 0; off < n && !s; off += chunk) {
     const size_t c = std::min(chunk, n - off);
@@ -1214,6 +1267,8 @@ int s615_run_batch(s615_ctx* ctx, int id, s615_batch* b, unsigned flags, void* s
   DevTable* t = find_table(ctx, id);
   if (!t) return S615_E_NOTABLE;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  const PlaneUse use(ctx);
+  note_capture(*t, st);
   const TableView tv = view_of(*t);
   // after the launches: an event that s615_batch_free waits on before the
   // batch's buffers go to the pool (the caller may free without a sync).  Not in

@@ -105,6 +105,7 @@ struct DevTable {
   void *d_plane = nullptr, *d_splane = nullptr, *d_eplane = nullptr;
   size_t plane_bytes = 0, splane_bytes = 0, eplane_bytes = 0;   // eplane_bytes 0: d_plane's
   u32 plane_lb = 0;
+  bool planes_captured = false;   // a captured launch reads them: kept until the table is freed
 };
 
 // The staged probe (staged.cu) reads a plane in slices; the largest may have
@@ -269,6 +270,10 @@ struct s615_ctx {
   bool run_busy = false;
   cudaStream_t aux = nullptr;   // fill_batch's own kernels
   cudaEvent_t last_run = nullptr;   // after the context's latest s615_run_batch
+  // calls between taking a table's view and their last launch with it (PlaneUse):
+  // no plane is given back meanwhile
+  std::mutex plane_mu;
+  int plane_users = 0;
   s615::StageSpace stage;
 };
 
@@ -295,6 +300,27 @@ void stage_free(HostStage& s);
 // freed batch buffers; true if either held anything.
 bool release_run_batch(s615_ctx* ctx);
 
+// Planes are a cache: an allocation that finds no room gives them all back (a table is
+// then probed through its cells alone), except those of captured launches, and unless
+// a call is using them.  True if any were.
+bool release_planes(s615_ctx* ctx);
+struct PlaneUse {
+  s615_ctx* ctx;
+  explicit PlaneUse(s615_ctx* c) : ctx(c) {
+    std::lock_guard<std::mutex> lock(ctx->plane_mu);
+    ++ctx->plane_users;
+  }
+  ~PlaneUse() {
+    std::lock_guard<std::mutex> lock(ctx->plane_mu);
+    --ctx->plane_users;
+  }
+  PlaneUse(const PlaneUse&) = delete;
+  PlaneUse& operator=(const PlaneUse&) = delete;
+};
+
+// What may still be allocated: the device's free bytes or what the budget leaves,
+// whichever is less.
+size_t hbm_room(const s615_ctx* ctx);
 // Budgeted device allocation.  dev_alloc_once neither gives anything back nor
 // tries again when there is no room.
 int dev_alloc_once(s615_ctx* ctx, void** p, size_t bytes);
@@ -333,6 +359,9 @@ int launch_peel(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flag
 int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                   cudaStream_t st, bool* done);
 void stage_release(s615_ctx* ctx);   // the caller holds ctx->stage.mu
+// The space that the least batch worth staging takes (with or without a one-bit plane
+// in front of the stages).
+size_t stage_least_bytes(u64 block, bool eplane);
 int launch_peel617(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                    cudaStream_t st, int grid_blocks);
 // Builds t's plane when it would make the probe cheaper (and the HBM budget

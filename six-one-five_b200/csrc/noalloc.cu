@@ -170,7 +170,10 @@ extern "C" int s615_cls5_run_noalloc(s615_ctx* ctx, int table_id, const s615_uni
   b.d_work = &S->work;
   b.item_rows = unit_rows;
   b.blocks_per_sm = tuned.blocks_per_sm;
-  if ((s = launch_peel(ctx, view_of(it->second), &b, flags, st, 0))) return s;
+  {
+    const PlaneUse use(ctx);
+    if ((s = launch_peel(ctx, view_of(it->second), &b, flags, st, 0))) return s;
+  }
 
   Cls5Counters c{};
   S615_CU(cudaMemcpyAsync(&c, &S->ctr, sizeof c, cudaMemcpyDeviceToHost, st));

@@ -327,7 +327,17 @@ Layout layout_for(u64 keys, u32 nb) {
   return L;
 }
 
+u32 stage_buckets(u64 block) {
+  const u32 sb = stage_shift(block);
+  return (u32)((block + (1ull << sb) - 1) >> sb);
+}
+constexpr double kSlack = 1.05;   // of the estimated keys
+
 }  // namespace
+
+size_t stage_least_bytes(u64 block, bool eplane) {
+  return layout_for((u64)(kMinKeys * kSlack / (eplane ? 2 : 1)), stage_buckets(block)).bytes;
+}
 
 void stage_release(s615_ctx* ctx) {
   StageSpace& w = ctx->stage;
@@ -358,15 +368,12 @@ int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned fl
   std::lock_guard<std::mutex> lock(ctx->stage.mu);
   StageSpace& w = ctx->stage;
   // chunks of at most kMaxChunkKeys keys, smaller when HBM is short
-  u64 keys = (u64)std::min<double>(est * 1.05, (double)kMaxChunkKeys);
+  u64 keys = (u64)std::min<double>(est * kSlack, (double)kMaxChunkKeys);
   const u32 sb = stage_shift(tv.block);
-  const u32 nb = (u32)((tv.block + (1ull << sb) - 1) >> sb);
+  const u32 nb = stage_buckets(tv.block);
   Layout L = layout_for(keys, nb);
   if (L.bytes > w.bytes) {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
-    const size_t used = ctx->used.load();
-    const size_t room = w.bytes + std::min(free_b, ctx->budget > used ? ctx->budget - used : 0) / 4;
+    const size_t room = w.bytes + hbm_room(ctx) / 4;
     while (L.bytes > room && keys > kMinChunkKeys) L = layout_for(keys = std::max(keys / 2, kMinChunkKeys), nb);
     if (L.bytes > w.bytes) {
       if (L.bytes > room) return S615_OK;

@@ -136,10 +136,16 @@ TableView view_of(const DevTable& t) {
   return v;
 }
 
+// Bytes of a plane of 2^lb bits of m cells: whole cells per 32-bit word.
+static size_t plane_size(u64 m, int lb) {
+  const u64 per = 32u >> lb;
+  return (m + per - 1) / per * sizeof(u32);
+}
+
 // 2^lb bits of t's cells, from bit `shift` on; *p stays null when there is no room.
 static int make_plane(s615_ctx* ctx, const DevTable& t, int lb, u32 shift, cudaStream_t st, void** p,
                       size_t* bytes) {
-  const u64 m = t.hdr.m_cells, per = 32u >> lb, words = (m + per - 1) / per;
+  const u64 m = t.hdr.m_cells, words = plane_size(m, lb) / sizeof(u32);
   if (dev_alloc_once(ctx, p, words * sizeof(u32))) return S615_OK;
   k_plane<<<grid_for(ctx, words, 256), 256, 0, st>>>(t.d_cells, (u32)t.layout, (u32)t.cell_bytes,
                                                      t.hdr.r, m, (u32)lb, shift,
@@ -191,6 +197,7 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
     const double ps = 3 * read_ps(mb) + cell_ps / (double)(1u << bits);
     if (mb <= kPlaneMaxMB && ps < best) { best = ps; lb = k; }
   }
+  // (Planes yield: an allocation that finds no room gives them back, release_planes.)
   if (lb >= 0) {
     if (const int s = make_plane(ctx, t, lb, 0, st, &t.d_plane, &t.plane_bytes)) return s;
     t.plane_lb = (u32)lb;
@@ -201,14 +208,23 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   if ((t.d_plane ? best : cell_ps) < kStagedFrom || t.bytes < ((size_t)1 << 28) || t.hdr.r < 16 ||
       m / 2 / 3 / 16 > kStageSlice)
     return S615_OK;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return S615_OK; }
-  if (4 * (m / 2) > free_b) return S615_OK;   // room that a search will want
-  if (m / 8 <= kEPlaneMax) {
-    if (t.d_plane && lb == 0) t.d_eplane = t.d_plane;
-    else if (const int s = make_plane(ctx, t, 0, 0, st, &t.d_eplane, &t.eplane_bytes)) return s;
+  // At most a quarter of the room that is left; and it is of use only to runs that
+  // find a quarter of what then remains enough for their keys (launch_staged's rule).
+  const bool one_bit = m / 8 <= kEPlaneMax, own = one_bit && !(t.d_plane && lb == 0);
+  const size_t want = plane_size(m, 2) + (own ? plane_size(m, 0) : 0);
+  const size_t room = hbm_room(ctx);
+  if (4 * want > room || 4 * stage_least_bytes(m / 3, one_bit) > room - want) return S615_OK;
+  if (own) {
+    if (const int s = make_plane(ctx, t, 0, 0, st, &t.d_eplane, &t.eplane_bytes)) return s;
+  } else if (one_bit) {
+    t.d_eplane = t.d_plane;
   }
-  return make_plane(ctx, t, 2, t.d_eplane ? 1u : 0u, st, &t.d_splane, &t.splane_bytes);
+  const int s = make_plane(ctx, t, 2, t.d_eplane ? 1u : 0u, st, &t.d_splane, &t.splane_bytes);
+  if (s || t.d_splane) return s;
+  if (own) dev_free(ctx, t.d_eplane, t.eplane_bytes);   // of no use alone
+  t.d_eplane = nullptr;
+  t.eplane_bytes = 0;
+  return S615_OK;
 }
 
 int launch_xor_query(s615_ctx* ctx, const TableView& tv, const u64* d_keys, size_t n,
