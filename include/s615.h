@@ -371,9 +371,14 @@ int s615_cls5_run(s615_ctx* ctx, int table_id, const s615_unit* units, size_t n,
 /* Device-resident form: the units are packed and uploaded once
  * (s615_prepare); each s615_run_batch is one or two launches on the caller's
  * stream (NULL = the context's stream), or for a large batch against a table
- * past L2 a sequence of launches there (with a space of up to a quarter of the
- * free HBM, kept and given back as s615_run's buffers are; not while the stream
- * is being captured); results stay on the device until
+ * past L2 a sequence of launches there.  That sequence works in a space of 5.0 GB
+ * (a quarter of the free HBM at most), which the first such run of a context
+ * allocates and the context keeps, and gives back as s615_run's buffers are; runs on
+ * two streams use it in turn.  Without it (no room, or the stream is being
+ * captured) the batch is one launch.  A space that little room made small is given up for
+ * a larger one only by a run that finds no other run of the context on the device.
+ * A captured launch reads the table's planes and the batch's buffers: free
+ * neither before the graph's last replay has ended.  Results stay on the device until
  * s615_batch_results.  s615_batch_free first waits for the batch's last
  * s615_run_batch to finish (it may be called right after the launch, with no
  * sync), then hands the batch's device buffers to a pool on the context (up to

@@ -990,7 +990,7 @@ static u32 tune_bucket(size_t n) {
 // whose persistent grid fills the SMs, they would wait for it to end, and a
 // caller (or the serving loop) that prepares a batch while another runs would
 // lose that overlap: then the host does the work.
-static bool device_idle(s615_ctx* ctx) {
+bool device_idle(s615_ctx* ctx) {
   if (serving(ctx)) return false;
   if (!ctx->last_run) return true;
   const cudaError_t e = cudaEventQuery(ctx->last_run);

@@ -213,12 +213,13 @@ struct s615_batch {
 
 namespace s615 {
 // The staged probe's key lists and chunk counters: one space per context, handed
-// from run to run (on any stream) through the event; given back with
-// s615_run's kept batch.
+// from run to run (on any stream) through the event, so staged runs on two streams
+// take turns; given back with s615_run's kept batch.
 struct StageSpace {
   std::mutex mu;
   void* p = nullptr;
   size_t bytes = 0;
+  u64 keys = 0;                 // a chunk's
   cudaEvent_t last = nullptr;   // recorded after the last run that used it
 };
 
@@ -291,6 +292,8 @@ int cuda_status(cudaError_t e);
 // its worker thread (calls that allocate or launch then return S615_E_BUSY).
 bool serving_blocks(s615_ctx* ctx);
 bool serving(const s615_ctx* ctx);    // true while a request loop owns the context
+// No run of the context is on the device, and no request loop would put one there.
+bool device_idle(s615_ctx* ctx);
 void server_destroy(s615_ctx* ctx);   // stops the loop (draining it) and frees it
 
 // Host staging (grow-only; nullptr if even a pageable buffer cannot be had).
@@ -361,7 +364,7 @@ int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned fl
 void stage_release(s615_ctx* ctx);   // the caller holds ctx->stage.mu
 // The space that the least batch worth staging takes (with or without a one-bit plane
 // in front of the stages).
-size_t stage_least_bytes(u64 block, bool eplane);
+size_t stage_least_bytes(bool eplane);
 int launch_peel617(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned flags,
                    cudaStream_t st, int grid_blocks);
 // Builds t's plane when it would make the probe cheaper (and the HBM budget

@@ -13,7 +13,9 @@
 //    others run join the next batch, and a batch is launched as soon as one of
 //    `slots` streams is free and its device buffers fit the HBM budget.
 //    Batches on different streams overlap on the device (a new persistent
-//    grid fills SMs as the previous one drains).
+//    grid fills SMs as the previous one drains); the staged parts of two large
+//    batches take turns in the context's one space for them, which the first of
+//    them allocates and no batch grows.
 //  * When a batch's event completes, its hits are verified and split back
 //    per request (unit indices rebased to the request); results wait for
 //    s615_poll and stay readable until s615_release.

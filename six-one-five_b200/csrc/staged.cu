@@ -326,18 +326,45 @@ Layout layout_for(u64 keys, u32 nb) {
   L.bytes = (sizeof(StageChunk) + 255) / 256 * 256 + L.first + L.second;
   return L;
 }
-
-u32 stage_buckets(u64 block) {
-  const u32 sb = stage_shift(block);
-  return (u32)((block + (1ull << sb) - 1) >> sb);
+// What a space for chunks of `keys` keys takes, whatever the table (layout_for rounds
+// each of at most kStageBuckets parts up by at most a piece).
+size_t space_bytes(u64 keys) {
+  return (sizeof(StageChunk) + 255) / 256 * 256 +
+         2 * 8 * ((size_t)(keys + keys / 8) + ((size_t)kStageBuckets << kStagePieceLog2));
 }
+
 constexpr double kSlack = 1.05;   // of the estimated keys
+
+// The context's space, for chunks of `want` keys, or of kMinChunkKeys at least; false:
+// there is no room.  It is taken at its largest useful size, a quarter of the room at
+// most, by the first run that wants one, so later runs neither allocate nor wait.
+// (Grown to each new largest batch, it was freed and allocated inside s615_run_batch,
+// behind the work in flight on every stream; and an allocation soon after the free
+// stalled: the first pass over the 155,391-unit band after a 300-unit one took 3,140 ms,
+// two times of three, where a pass takes 2,530.)  A space that little room made smaller
+// is given up for a larger one only when nothing has to be waited for.
+bool take_space(s615_ctx* ctx, u64 want) {
+  StageSpace& w = ctx->stage;
+  const u64 least = std::min(want, kMinChunkKeys);
+  if (w.p && (w.keys >= want || !device_idle(ctx))) return w.keys >= least;
+  const size_t room = w.bytes + hbm_room(ctx) / 4;
+  u64 keys = kMaxChunkKeys;
+  while (space_bytes(keys) > room && keys > kMinChunkKeys) keys /= 2;
+  if (space_bytes(keys) > room) keys = least;
+  if (keys <= w.keys) return w.keys >= least;
+  if (space_bytes(keys) > room) return false;
+  stage_release(ctx);
+  void* p = nullptr;
+  if (dev_alloc_once(ctx, &p, space_bytes(keys))) return false;
+  w.p = p;
+  w.bytes = space_bytes(keys);
+  w.keys = keys;
+  return true;
+}
 
 }  // namespace
 
-size_t stage_least_bytes(u64 block, bool eplane) {
-  return layout_for((u64)(kMinKeys * kSlack / (eplane ? 2 : 1)), stage_buckets(block)).bytes;
-}
+size_t stage_least_bytes(bool eplane) { return space_bytes((u64)(kMinKeys * kSlack / (eplane ? 2 : 1))); }
 
 void stage_release(s615_ctx* ctx) {
   StageSpace& w = ctx->stage;
@@ -349,6 +376,7 @@ void stage_release(s615_ctx* ctx) {
   dev_free(ctx, w.p, w.bytes);
   w.p = nullptr;
   w.bytes = 0;
+  w.keys = 0;
 }
 
 // *done = true when the classes 2-5 items of b were probed in stages.
@@ -368,22 +396,12 @@ int launch_staged(s615_ctx* ctx, const TableView& tv, s615_batch* b, unsigned fl
   std::lock_guard<std::mutex> lock(ctx->stage.mu);
   StageSpace& w = ctx->stage;
   // chunks of at most kMaxChunkKeys keys, smaller when HBM is short
-  u64 keys = (u64)std::min<double>(est * kSlack, (double)kMaxChunkKeys);
+  const u64 want = (u64)std::min<double>(est * kSlack, (double)kMaxChunkKeys);
+  if (!take_space(ctx, want)) return S615_OK;
+  const u64 keys = std::min(want, w.keys);
   const u32 sb = stage_shift(tv.block);
-  const u32 nb = stage_buckets(tv.block);
-  Layout L = layout_for(keys, nb);
-  if (L.bytes > w.bytes) {
-    const size_t room = w.bytes + hbm_room(ctx) / 4;
-    while (L.bytes > room && keys > kMinChunkKeys) L = layout_for(keys = std::max(keys / 2, kMinChunkKeys), nb);
-    if (L.bytes > w.bytes) {
-      if (L.bytes > room) return S615_OK;
-      stage_release(ctx);
-      void* p = nullptr;
-      if (dev_alloc_once(ctx, &p, L.bytes)) return S615_OK;
-      w.p = p;
-      w.bytes = L.bytes;
-    }
-  }
+  const u32 nb = (u32)((tv.block + (1ull << sb) - 1) >> sb);
+  const Layout L = layout_for(keys, nb);
   if (!w.last) S615_CU(cudaEventCreateWithFlags(&w.last, cudaEventDisableTiming));
   else S615_CU(cudaStreamWaitEvent(st, w.last, 0));   // the space's last user, on any stream
   *done = true;

@@ -213,7 +213,7 @@ int build_plane(s615_ctx* ctx, DevTable& t, cudaStream_t st) {
   const bool one_bit = m / 8 <= kEPlaneMax, own = one_bit && !(t.d_plane && lb == 0);
   const size_t want = plane_size(m, 2) + (own ? plane_size(m, 0) : 0);
   const size_t room = hbm_room(ctx);
-  if (4 * want > room || 4 * stage_least_bytes(m / 3, one_bit) > room - want) return S615_OK;
+  if (4 * want > room || 4 * stage_least_bytes(one_bit) > room - want) return S615_OK;
   if (own) {
     if (const int s = make_plane(ctx, t, 0, 0, st, &t.d_eplane, &t.eplane_bytes)) return s;
   } else if (one_bit) {
