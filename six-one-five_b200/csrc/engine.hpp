@@ -321,6 +321,17 @@ struct PlaneUse {
   PlaneUse& operator=(const PlaneUse&) = delete;
 };
 
+// Allocating and freeing are refused, and spoil the capture, while a stream is being
+// captured in the global mode (the default), whatever stream they are for.  In this
+// scope the calling thread's such calls leave other streams' captures alone.
+struct CaptureRelaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  CaptureRelaxed(const CaptureRelaxed&) = delete;
+  CaptureRelaxed& operator=(const CaptureRelaxed&) = delete;
+};
+
 // What may still be allocated: the device's free bytes or what the budget leaves,
 // whichever is less.
 size_t hbm_room(const s615_ctx* ctx);

@@ -346,6 +346,7 @@ constexpr double kSlack = 1.05;   // of the estimated keys
 bool take_space(s615_ctx* ctx, u64 want) {
   StageSpace& w = ctx->stage;
   const u64 least = std::min(want, kMinChunkKeys);
+  const CaptureRelaxed relaxed;
   if (w.p && (w.keys >= want || !device_idle(ctx))) return w.keys >= least;
   const size_t room = w.bytes + hbm_room(ctx) / 4;
   u64 keys = kMaxChunkKeys;

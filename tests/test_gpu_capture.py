@@ -57,3 +57,56 @@ def test_freeing_a_captured_batch(engine):
         assert [getattr(c, f) for f in FIELDS] == want[0] and len(h) == len(want[1])
     finally:
         engine.free_table(tid)
+
+
+@pytest.fixture(scope="module")
+def staged():
+    """A table whose large batches are probed in stages, and such a batch's units."""
+    N = 40000
+    arr, n = W.unit_array(W.cls5_units(1650000, 1650600)[:1500], W.plants(2, 5, 1600000, 1680000, N), N)
+    with s615.Engine(0) as eng:
+        yield eng, eng.build_table(N, 20), arr, n
+
+
+def give_space_back(eng):
+    eng.free_table(eng.build_table(300, 16))
+
+
+def test_beside_a_capture(staged):
+    """The first staged run of a context while another stream is captured in the default
+    (global) mode: the capture stays valid, and the run is staged."""
+    eng, tid, arr, n = staged
+    p, st = prepare(eng, arr, n), torch.cuda.Stream()
+    launch(eng, tid, p, st)                   # kernels loaded
+    torch.cuda.synchronize()
+    want = results(eng, p)
+    give_space_back(eng)
+    x, g = torch.ones(1000, device="cuda"), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        y = x + 1
+        launched = launch(eng, tid, p, st)
+    g.replay()
+    torch.cuda.synchronize()
+    assert launched >= 5 and float(y.sum()) == 2000
+    assert results(eng, p) == want
+    s615.lib().s615_batch_free(eng._ctx, p)
+
+
+def test_a_captured_run_is_direct(staged):
+    """A run on a stream that is being captured goes without the space, and its replay
+    gives the staged run's results."""
+    eng, tid, arr, n = staged
+    p, st = prepare(eng, arr, n), torch.cuda.Stream()
+    assert launch(eng, tid, p, st) >= 5
+    torch.cuda.synchronize()
+    want, g = results(eng, p), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        assert launch(eng, tid, p, st) <= 2
+    give_space_back(eng)
+    for _ in range(2):
+        g.replay()
+    torch.cuda.synchronize()
+    assert results(eng, p) == want
+    del g
+    s615.lib().s615_batch_free(eng._ctx, p)
