@@ -136,10 +136,8 @@ struct TableView {
   u64 shard_seed;
   u32 grp_lo, grp_hi;   // this pass probes keys of shards [grp_lo, grp_hi)
   u32 groups, pad;      // passes over the set
-  u64 bytes;            // bytes of cells (a single table; 0 for a set)
   const u32* plane;     // low 2^plane_lb bits of each cell (null: none)
   const u32 *splane, *eplane;   // the staged probe's
-  u64 plane_bytes;
   u32 plane_lb, plane_mask;   // plane_mask = 2^(2^plane_lb) - 1
 };
 

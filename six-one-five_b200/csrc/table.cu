@@ -118,7 +118,6 @@ TableView view_of(const DevTable& t) {
     return v;
   }
   v.cells = t.d_cells;
-  v.bytes = t.bytes;
   v.block = t.hdr.m_cells / 3;
   v.recip = mod_recip(v.block);
   v.fpmask = fp_mask(t.hdr.r);
@@ -129,7 +128,6 @@ TableView view_of(const DevTable& t) {
   v.plane = static_cast<const u32*>(t.d_plane);
   v.splane = static_cast<const u32*>(t.d_splane);
   v.eplane = static_cast<const u32*>(t.d_eplane);
-  v.plane_bytes = t.plane_bytes;
   v.plane_lb = t.plane_lb;
   v.plane_mask = (u32)((1ull << (1u << t.plane_lb)) - 1);
   if (t.hdr.n_keys == 0 || t.hdr.m_cells < 3) v.block = 0;
