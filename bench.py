@@ -45,6 +45,7 @@ METRIC = "cls5 peel probes/sec and eligible-B/hour at B≈3.2M, 1 B200; p99 unit
 UNIT = "peel_probes/s"
 BAND_LO, BAND_W = 3_200_000, 20_000
 PROBE_BYTES = 108          # 3 cells x 1.125 sectors x 32 B per post-gate xor probe (r=48)
+STAGED_LAUNCHES = 6        # launches a chunk of the staged probe: emit, steps 0 to 3, resolve
 N_PLANTS = 32
 
 
@@ -179,15 +180,50 @@ def probe_only_ceiling(lib, eng, tid, stream, n=1 << 28):
     return 3 * n / (best / 1e3), best
 
 
-def random_access_roof(lib, eng, tid, stream, probes, dur_s):
-    """The probe's binding roofline: the pass's cell reads/s (3 per post-gate
-    probe) over the probe-only ceiling on the same table."""
-    ceil, ms = probe_only_ceiling(lib, eng, tid, stream)
-    got = 3 * probes / dur_s
-    return {"achieved_reads_per_s": got, "ceiling_reads_per_s": ceil,
-            "frac": round(got / ceil, 4) if ceil else None,
-            "ceiling_source": "k_xor_query (s615_xor_query_dev) on 2^28 uniformly random keys against "
-                              f"the same resident table, same process, after the timed region: {ms:.2f} ms"}
+def roofline(lib, eng, tid, stream, probes, dur_s, launches):
+    """The probe's roofline for one launch of `launches` kernels that took dur_s, by the path
+    that the post-gate keys took (told from the launches and the table's planes).  The bytes
+    are counted, not measured: that needs a profiler, and the run has none.
+
+      direct: three cells a key from HBM, 108 B in sectors.  What binds it is the rate of
+              scattered reads, so the pass's cell reads/s are set beside the same table's
+              probe-only rate (random_access; one table only).
+      plane:  three 32-byte sectors a key from a plane that stays in L2, and for one key in
+              2^bits the cells.
+      staged: a key's 8-byte entry written and read between the steps (64 B), for one key in
+              16 three 64-byte fills of its cells (12 B), and the 4-bit plane once a chunk.
+              With a one-bit plane in front, half of the keys."""
+    info = eng.table_info(tid)
+    m, r, single = info.hdr.m_cells, info.hdr.r, info.hdr.shard_count == 1
+    cells = m * info.cell_bytes if info.cell_bytes else ((m * r + 7) // 8 + 15) // 8 * 8 + 8
+    peak, kind = measured_peaks()
+    roof = {"bound": "hbm", "peak": peak, "unit": "GB/s", "peak_kind": f"{kind} hbm_gbs (burst)",
+            "traffic": None, "bytes_kind": "counted by path, not measured"}
+    if single and launches >= STAGED_LAUNCHES:
+        keys = probes / 2 if m / 8 <= 60 << 20 else probes
+        roof["path"] = "staged"
+        total = 76 * keys + (launches // STAGED_LAUNCHES) * m / 2
+    elif single and info.device_bytes > cells and m / 8 <= 112 << 20:
+        bits = round((info.device_bytes - cells) * 8 / m)
+        bits = {5: 1, 6: 2, 7: 2}.get(bits, bits)   # the staged probe's planes beside it
+        roof.update(path="plane", bound="l2", peak=None, peak_kind=None)
+        total = probes * (96 + PROBE_BYTES / 2 ** bits)
+    else:
+        roof["path"] = "direct"
+        total = probes * PROBE_BYTES
+        if single:
+            ceil, ms = probe_only_ceiling(lib, eng, tid, stream)
+            got = 3 * probes / dur_s
+            roof["random_access"] = {
+                "achieved_reads_per_s": got, "ceiling_reads_per_s": ceil,
+                "frac": round(got / ceil, 4) if ceil else None,
+                "ceiling_source": "k_xor_query (s615_xor_query_dev) on 2^28 uniformly random keys "
+                                  "against the same resident table, same process, after the timed "
+                                  f"region: {ms:.2f} ms"}
+    got = total / dur_s / 1e9
+    roof.update(achieved=round(got, 1), frac=round(got / peak, 4) if roof["peak"] else None,
+                algorithmic_bytes_per_launch=int(total), bytes_per_key=round(total / max(probes, 1), 1))
+    return roof
 
 
 def log(msg):
@@ -584,14 +620,10 @@ def run617(args, rank, world, local, dist):
     if rank == 0 and not args.no_find4:
         find4 = run617_find4(lib, eng, tid, stream, Bs)
 
-    peak, peak_kind = measured_peaks()
-    achieved = ctr.probes * PROBE_BYTES / (statistics.mean(per_ms) / 1e3) / 1e9
-    roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "peak_kind": f"{peak_kind} hbm_gbs (burst)",
-            "traffic": None, "algorithmic_bytes_per_launch": ctr.probes * PROBE_BYTES}
+    roof = None
     if rank == 0:
-        roof["random_access"] = random_access_roof(lib, eng, tid, stream, ctr.probes,
-                                                   statistics.mean(per_ms) / 1e3)
+        roof = roofline(lib, eng, tid, stream, ctr.probes, statistics.mean(per_ms) / 1e3,
+                        launches // args.steps)
 
     cpu = None
     if not args.no_cpu_baseline and rank == 0 and world == 1:
@@ -764,8 +796,8 @@ def solve_516_cfg1(points, runs=15):
 def run_cfg1(args, rank, world, local, dist):
     """--workload cfg1: the small CPU-runnable configuration -- every class-5
     unit of B in [1000, 30000] (725) plus 8 plants against an N = 715, r = 48
-    table built on the device (1.9 MB) -- timed with and without the peel's
-    S615_F_NO_L2_WINDOW (which has no effect any more), and the oracle on the host cores beside it."""
+    table built on the device (1.9 MB) -- timed, and
+    the oracle on the host cores beside it."""
     import numpy as np
     import torch
 
@@ -785,12 +817,10 @@ def run_cfg1(args, rank, world, local, dist):
     b = C.c_void_p()
     s615._check(lib.s615_prepare(eng._ctx, C.cast(arr, C.c_void_p), n, C.byref(b)), "prepare")
     stream = torch.cuda.Stream()
-    res = {}
-    for name, fl in (("window", 0), ("no_window", s615.F_NO_L2_WINDOW)):
-        for _ in range(args.warmup):
-            timed_steps(lib, eng, tid, b, stream, fl, 1)
-        ms, c = timed_steps(lib, eng, tid, b, stream, fl, max(args.steps, 50))
-        res[name] = {"ms_per_pass": ms / max(args.steps, 50), "pos": c.pos, "probes": c.probes}
+    steps = max(args.steps, 50)
+    for _ in range(args.warmup):
+        timed_steps(lib, eng, tid, b, stream, 0, 1)
+    ms, c = timed_steps(lib, eng, tid, b, stream, 0, steps)
     s615._check(lib.s615_batch_free(eng._ctx, b), "batch_free")
     hb, pk = eng.export_table(tid)
     ot = orc.Table.from_memory(hb, pk)
@@ -802,14 +832,14 @@ def run_cfg1(args, rank, world, local, dist):
     port = {"value": (gated + probes) / cpu_s, "unit": UNIT, "cores": os.cpu_count(),
             "kind": "port", "sample": f"all {len(units)} units once"}
     ref = solve_516_cfg1(gated + probes)
-    v = res["window"]["pos"] / (res["window"]["ms_per_pass"] / 1e3)
+    v = c.pos * steps / (ms / 1e3)
     line = {"metric": "cls5 peel probes/sec, B in [1000, 30000] (config 1), 1 B200", "value": v,
-            "unit": UNIT, "n_gpus": 1, "steps": max(args.steps, 50), "warmup": args.warmup,
-            "ms_per_step": res["window"]["ms_per_pass"], "higher_is_better": True, "scaling": "weak",
+            "unit": UNIT, "n_gpus": 1, "steps": steps, "warmup": args.warmup,
+            "ms_per_step": ms / steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "u64", "data": "synthetic",
             "config": {"workload": f"config 1: {len(units)} Stage-1 units + 8 plants, N={N} r={args.r} "
                                    "table built on the device (1.9 MB: fits L2)"},
-            "l2_window": res,
+            "counters": {"probes": c.probes, "pos": c.pos},
             "cpu_baseline": ref or port,
             "cpu_port": port}
     print(json.dumps(line), flush=True)
@@ -883,14 +913,10 @@ def run_mix(args, rank, world, local, dist):
     e2e_ms, e2e_job = shard.merge(dist, "cuda", e2e_s * 1e3, {"units": n})
     step_s = job_ms / args.steps / 1e3
     # the probe's roofline for one launch (all steps are the same pass)
-    peak, peak_kind = measured_peaks()
-    per_s = (ms / args.steps) / 1e3
-    achieved = ctr.probes * PROBE_BYTES / per_s / 1e9
-    mix_roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                "frac": round(achieved / peak, 4), "peak_kind": f"{peak_kind} hbm_gbs (burst)",
-                "traffic": None, "algorithmic_bytes_per_launch": ctr.probes * PROBE_BYTES,
-                "random_access": random_access_roof(lib, eng, tid, stream, ctr.probes, per_s)
-                if rank == 0 else None}
+    mix_roof = None
+    if rank == 0:
+        mix_roof = roofline(lib, eng, tid, stream, ctr.probes, ms / args.steps / 1e3,
+                            launches // args.steps)
     line = {"metric": METRIC_MIX, "value": job["units"] / step_s, "unit": "units/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": job_ms / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u64",
@@ -1069,8 +1095,6 @@ def run_jobs(args, rank, world, local, dist):
     total_ms, tot = shard.merge(dist, "cuda", total_ms, {"jobs": n})
     e2e_ms, e2e_job = shard.merge(dist, "cuda", e2e_s * 1e3, {"jobs": n})
     step_s = total_ms / args.steps / 1e3
-    peak, peak_kind = measured_peaks()
-    achieved = ctr.probes * PROBE_BYTES / (statistics.mean(per_ms) / 1e3) / 1e9
     mix = collections.Counter(c for c, _, _ in units)
     jmix = collections.Counter(jobs[i].cls for i in range(0, n, max(1, n // 100000)))
     line = {"metric": METRIC_JOBS, "value": tot["jobs"] / step_s, "unit": "jobs/s", "n_gpus": world,
@@ -1096,12 +1120,8 @@ def run_jobs(args, rank, world, local, dist):
                     "d2h_bytes_per_step": C.sizeof(s615.Counters) + len(h3) * C.sizeof(s615.Hit),
                     "includes": ".bbj read + s615_run", "phases": e2e_phases},
             "gpu_launches": launches,
-            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                         "frac": round(achieved / peak, 4), "peak_kind": f"{peak_kind} hbm_gbs (burst)",
-                         "traffic": None, "algorithmic_bytes_per_launch": ctr.probes * PROBE_BYTES,
-                         "random_access": (random_access_roof(
-                             lib, eng, tid, stream, ctr.probes, statistics.mean(per_ms) / 1e3)
-                             if rank == 0 else None)},
+            "roofline": (roofline(lib, eng, tid, stream, ctr.probes, statistics.mean(per_ms) / 1e3,
+                                  launches // args.steps) if rank == 0 else None),
             "cpu_baseline": cpu, "sharp_gate": sharp, "clocks": cl}
     eng.close()
     if rank == 0:
@@ -1388,6 +1408,8 @@ def main():
         t0 = time.perf_counter()
         b2 = C.c_void_p()
         s615._check(lib.s615_prepare(eng._ctx, C.cast(arr, C.c_void_p), n, C.byref(b2)), "prepare")
+        # this one allocates the batch's buffers (a cudaMalloc can stall for hundreds of ms on
+        # a fresh machine); the later ones find them in the context's pool
         ph["prepare_ms"] = (time.perf_counter() - t0) * 1e3
         t0 = time.perf_counter()
         s615._check(lib.s615_run_batch(eng._ctx, tid, b2, 0, None), "run_batch")
@@ -1399,33 +1421,21 @@ def main():
         t0 = time.perf_counter()
         s615._check(lib.s615_batch_free(eng._ctx, b2), "batch_free")
         ph["free_ms"] = (time.perf_counter() - t0) * 1e3
+        t0 = time.perf_counter()
+        s615._check(lib.s615_prepare(eng._ctx, C.cast(arr, C.c_void_p), n, C.byref(b2)), "prepare")
+        ph["prepare_again_ms"] = (time.perf_counter() - t0) * 1e3
+        s615._check(lib.s615_batch_free(eng._ctx, b2), "batch_free")
         e2e_phases = {k: round(v, 1) for k, v in ph.items()}
         e2e_phases["note"] = ("a fresh batch through s615_prepare / s615_run_batch / "
                               "s615_batch_free; s615_cls5_run reuses the context's kept batch")
         log(f"e2e phases: {e2e_phases}")
 
-    peak, peak_kind = measured_peaks()
-    dur_s = statistics.mean(per_ms) / 1e3
-    achieved = ctr.probes * PROBE_BYTES / dur_s / 1e9
-    roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "peak_kind": f"{peak_kind} hbm_gbs (burst)",
-            # DRAM bytes need a profiler; this run has none (the ncu capture of the
-            # same pass is summarised beside the kernel's roofline in the design notes)
-            "traffic": None,
-            "algorithmic_bytes_per_launch": ctr.probes * PROBE_BYTES}
-    if rank == 0 and args.shards == 1:
-        roof["random_access"] = random_access_roof(lib, eng, tid, stream, ctr.probes, dur_s)
-        log("random-access roofline: %.3e cell reads/s of %s measured (%s)" % (
-            roof["random_access"]["achieved_reads_per_s"],
-            "%.3e" % roof["random_access"]["ceiling_reads_per_s"]
-            if roof["random_access"]["ceiling_reads_per_s"] else "n/a",
-            roof["random_access"]["frac"]))
-    # DRAM bytes the staged probe moves per post-gate key: eight passes of its 8-byte
-    # entry (written and read between the steps) and, for one key in 16, three 64-byte
-    # fills of its cells; against the same copy peak
-    dram = 76 * ctr.probes / dur_s / 1e9
-    roof["dram_fills"] = {"bytes_per_key": 76, "achieved": round(dram, 1), "peak": peak,
-                          "unit": "GB/s", "frac": round(dram / peak, 4)}
+    roof = None
+    if rank == 0:
+        roof = roofline(lib, eng, tid, stream, ctr.probes, statistics.mean(per_ms) / 1e3,
+                        launches // args.steps)
+        log(f"roofline: {roof['path']} probe, {roof['bytes_per_key']} B a key, "
+            f"{roof['achieved']} GB/s")
 
     # plain per-unit-launch form on a bounded sample of the same band
     plain = None
@@ -1534,7 +1544,6 @@ def main():
                    "shards": args.shards,
                    "units_per_rank": n, "N": N, "r": args.r,
                    "l2": "inputs larger than L2 (table %.1f GB)" % (eng.table_info(tid).device_bytes / 1e9),
-                   "l2_window": False,
                    "parallelism": (f"shard-split x{world}: each rank holds {args.shards // world}+ of "
                                    f"{args.shards} shards and runs the whole band" if split
                                    else f"replicas-by-band x{world}")},
