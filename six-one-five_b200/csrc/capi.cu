@@ -1199,9 +1199,11 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   // long list is put in that order on the device, on its way into place.
   const size_t n617 = total - at[nt];
   const bool order_on_device = n617 > kOrderOnDevice && device_idle(ctx);
-  if (!order_on_device)
+  const auto order_on_host = [&]() {
     std::stable_sort(items + at[nt], items + total,
                      [](u64 a, u64 c) { return item_chunk(a) < item_chunk(c); });
+  };
+  if (!order_on_device) order_on_host();
   nvtxRangePop();
   NvtxRange upload("upload batch");
   b->n_units = nd;
@@ -1211,10 +1213,16 @@ int fill_batch(s615_ctx* ctx, const s615_unit* units, size_t n, s615_batch* b) {
   if (const int s = batch_buffers(ctx, b, nd, total)) return s;
   if (nd)
     S615_CU(cudaMemcpy(b->d_units, du, nd * sizeof(DevUnit), cudaMemcpyHostToDevice));
-  const size_t n_plain = order_on_device ? b->n_main : b->n_items;
+  size_t n_plain = b->n_items;   // items that go up as they are
+  if (order_on_device) {
+    const int s = upload_ordered(ctx, b);
+    if (s == S615_OK) n_plain = b->n_main;
+    else if (s == S615_E_OOM) order_on_host();   // no room for a second copy of them
+    else return s;
+  }
   if (n_plain)
     S615_CU(cudaMemcpy(b->d_items, b->host_items.get(), n_plain * sizeof(u64), cudaMemcpyHostToDevice));
-  return order_on_device ? upload_ordered(ctx, b) : S615_OK;
+  return S615_OK;
 }
 
 }  // namespace s615
