@@ -21,7 +21,7 @@ constexpr u32 kBloomBits = 19;             // positives of a chunk: 2^19 bits, 6
 constexpr u32 kStagePieceLog2 = 18;
 struct StageRuns {
   unsigned long long* e;
-  u32* count;              // [nb * kStageStride] (may pass cap: the rest were refused)
+  u32* count;              // [nb * kStageStride] (may pass cap: those keys were refused)
   u32 nb, cap;             // entries of a bucket
   __host__ __device__ __forceinline__ u64 at(u32 b, u32 i) const {
     return (((u64)(i >> kStagePieceLog2) * nb + b) << kStagePieceLog2) |
@@ -106,12 +106,19 @@ struct WarpHold {
 };
 
 // Appends the first n held keys; `direct(e)` probes a key that the list has no
-// room for.  All lanes call this.
+// room for.  All lanes call this.  A full list's counter is put back, so it stays
+// within what the warps add at once past the list's end.  Items are dealt to chunks by
+// number, and a chunk of the heaviest ones can hold hundreds of times the keys it was
+// sized for: with 2^32 for one list the counter would wrap and the list's keys be
+// overwritten.
 template <class Direct>
 __device__ __forceinline__ void stage_append(const StageRuns& O, u32 list, const WarpHold& H, u32 n,
                                              u32 lane, Direct direct) {
   u32 i0 = 0;
-  if (lane == 0) i0 = atomicAdd(O.count + list * kStageStride, n);
+  if (lane == 0) {
+    i0 = atomicAdd(O.count + list * kStageStride, n);
+    if (i0 >= O.cap) atomicSub(O.count + list * kStageStride, n);
+  }
   i0 = __shfl_sync(0xFFFFFFFFu, i0, 0);
 #pragma unroll 4
   for (u32 p = lane; p < n; p += 32) {
